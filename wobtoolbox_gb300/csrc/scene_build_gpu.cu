@@ -6,16 +6,20 @@
 // nondecreasing), guide tables, padded boxes -- with a different BVH topology: Morton codes of the
 // element centroids, a bitonic sort of (code, caller index), a binary radix tree over the sorted
 // codes (Karras, "Maximizing parallelism in the construction of BVHs, octrees, and k-d trees",
-// HPG 2012), bottom-up boxes, and a top-down collapse into the 4-wide layout (each wide node takes
-// its binary node's two children, each expanded once more when it holds more than kLeafMax
-// elements). Storage order is the sorted order, so every leaf is a contiguous range and a
-// depth-first traversal with children in order still returns hits in storage order; hit sets do
-// not depend on the topology. The CDFs are computed by one thread in storage order with the host
-// build's float operations (built with -fmad=false), so the sampling tables are bit-identical to a
-// host build over the same storage order.
+// HPG 2012), bottom-up boxes, and a collapse into the 4-wide layout (each wide node takes its binary
+// node's two children, each expanded once more when it holds more than kLeafMax elements: the wide
+// nodes are the binary nodes of even depth with more than kLeafMax elements, numbered in binary node
+// order). Storage order is the sorted order, so every leaf is a contiguous range and a depth-first
+// traversal with children in order still returns hits in storage order; hit sets do not depend on
+// the topology. Nothing is read back before the end: the checks of the input, the node count, the
+// depth and the totals come in one copy. The CDFs come from k_kahan.cu, whose prefix sums have the bits of the
+// host build's serial ones, so the sampling tables are bit-identical to a host build over the same
+// storage order.
 #include "scene_build_gpu.hpp"
 
+#include "kahan_scan.hpp"
 #include "scene_host.hpp"
+#include "sort_keys.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -40,57 +44,106 @@ __host__ __device__ inline float unord(uint32_t u) {
     return f;
 }
 
+constexpr uint32_t kBadTree = 64u;
+
 struct Bounds {  // ordered-uint encodings
     uint32_t lo[3], hi[3], clo[3], chi[3], mag;
-    uint32_t bad;            // bit 0 non-finite vertex, 1 normal, 2 data, 3 alpha, 4 type, 5 normal length
+    uint32_t bad;            // bit 0 non-finite vertex, 1 normal, 2 data, 3 alpha, 4 type, 5 normal length, 6 tree
     uint32_t all_dirichlet;  // 1 until a non-Dirichlet element is seen
+    uint32_t n_nodes, depth; // of the 4-wide tree
+    float totals[2];         // area, |g|
 };
+
+// padding of the host build: 1e-5 (extent + max |coordinate|)
+__host__ __device__ inline float box_pad(const Bounds &b, int dim) {
+    float ext = 0.0f;
+    for (int k = 0; k < dim; k++) {
+        const float e = unord(b.hi[k]) - unord(b.lo[k]);
+        ext = ext < e ? e : ext;
+    }
+    return 1e-5f * (ext + unord(b.mag)) + 1e-30f;
+}
 
 __device__ __forceinline__ bool finite_f(float x) { return isfinite(x); }
 
+// The checks of the input, element boxes and the scene's bounds. The bounds are reduced over the block
+// before the global atomics: one atomic an element and word on a handful of addresses took 0.35 ms
+// for 327,680 triangles, one a block 0.02 ms.
 template <int D>
-__global__ void k_validate(uint32_t n, const float *__restrict__ verts, const float *__restrict__ normals,
-                           const float *__restrict__ bvals, const float *__restrict__ alphas,
-                           const int32_t *__restrict__ types, float *__restrict__ box, Bounds *b) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t bad = 0;
-    const float *v = verts + (size_t)i * D * D;
-    for (int k = 0; k < D * D; k++)
-        if (!finite_f(v[k])) bad |= 1u;
-    for (int k = 0; k < D; k++) {
-        if (!finite_f(normals[(size_t)i * D + k])) bad |= 2u;
-        if (!finite_f(bvals[(size_t)i * D + k])) bad |= 4u;
-        if (alphas && !finite_f(alphas[(size_t)i * D + k])) bad |= 8u;
-    }
-    float q = 0.0f;
-    for (int k = 0; k < D; k++) q += normals[(size_t)i * D + k] * normals[(size_t)i * D + k];
-    if (!(q >= 0.25f && q <= 4.0f)) bad |= 32u;  // as the host build: normals far from unit length
-    const int t = types[i];
-    if (t < 0 || t > 2) bad |= 16u;
-    if (bad) atomicOr(&b->bad, bad);
-    if (t != 0) atomicAnd(&b->all_dirichlet, 0u);
-    // element box, centroid (scene_build.cpp: lo / hi / s / dim, left to right)
-    for (int k = D; k < 3; k++) box[(size_t)i * 9 + k] = box[(size_t)i * 9 + 3 + k] = box[(size_t)i * 9 + 6 + k] = 0.0f;
-    float mag = 0.0f;
-    for (int k = 0; k < D; k++) {
-        float lo = v[k], hi = v[k], s = v[k];
-        for (int j = 1; j < D; j++) {
-            lo = fminf(lo, v[j * D + k]);
-            hi = fmaxf(hi, v[j * D + k]);
-            s = s + v[j * D + k];
+__global__ void __launch_bounds__(kT) k_validate(uint32_t n, const float *__restrict__ verts,
+                                                 const float *__restrict__ normals, const float *__restrict__ bvals,
+                                                 const float *__restrict__ alphas, const int32_t *__restrict__ types,
+                                                 float *__restrict__ box, Bounds *b) {
+    constexpr int kWords = 4 * D + 1;  // per axis min lo, max hi, min c, max c; then max |coordinate|
+    __shared__ uint32_t red[kT / 32][kWords];
+    __shared__ uint32_t s_bad, s_other;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_bad = s_other = 0u;
+    __syncthreads();
+    uint32_t word[kWords];  // minima as complements, so that every word is a maximum
+#pragma unroll
+    for (int k = 0; k < kWords; k++) word[k] = 0u;
+    if (i < n) {
+        uint32_t bad = 0;
+        const float *v = verts + (size_t)i * D * D;
+        for (int k = 0; k < D * D; k++)
+            if (!finite_f(v[k])) bad |= 1u;
+        for (int k = 0; k < D; k++) {
+            if (!finite_f(normals[(size_t)i * D + k])) bad |= 2u;
+            if (!finite_f(bvals[(size_t)i * D + k])) bad |= 4u;
+            if (alphas && !finite_f(alphas[(size_t)i * D + k])) bad |= 8u;
         }
-        const float c = s / (float)D;
-        box[(size_t)i * 9 + k] = lo;
-        box[(size_t)i * 9 + 3 + k] = hi;
-        box[(size_t)i * 9 + 6 + k] = c;
-        atomicMin(&b->lo[k], ord(lo));
-        atomicMax(&b->hi[k], ord(hi));
-        atomicMin(&b->clo[k], ord(c));
-        atomicMax(&b->chi[k], ord(c));
-        mag = fmaxf(mag, fmaxf(fabsf(lo), fabsf(hi)));
+        float q = 0.0f;
+        for (int k = 0; k < D; k++) q += normals[(size_t)i * D + k] * normals[(size_t)i * D + k];
+        if (!(q >= 0.25f && q <= 4.0f)) bad |= 32u;  // as the host build: normals far from unit length
+        const int t = types[i];
+        if (t < 0 || t > 2) bad |= 16u;
+        if (bad) atomicOr(&s_bad, bad);
+        if (t != 0) s_other = 1u;
+        // element box, centroid (scene_build.cpp: lo / hi / s / dim, left to right)
+        for (int k = D; k < 3; k++)
+            box[(size_t)i * 9 + k] = box[(size_t)i * 9 + 3 + k] = box[(size_t)i * 9 + 6 + k] = 0.0f;
+        float mag = 0.0f;
+#pragma unroll
+        for (int k = 0; k < D; k++) {
+            float lo = v[k], hi = v[k], s = v[k];
+            for (int j = 1; j < D; j++) {
+                lo = fminf(lo, v[j * D + k]);
+                hi = fmaxf(hi, v[j * D + k]);
+                s = s + v[j * D + k];
+            }
+            const float c = s / (float)D;
+            box[(size_t)i * 9 + k] = lo;
+            box[(size_t)i * 9 + 3 + k] = hi;
+            box[(size_t)i * 9 + 6 + k] = c;
+            word[4 * k] = ~ord(lo);
+            word[4 * k + 1] = ord(hi);
+            word[4 * k + 2] = ~ord(c);
+            word[4 * k + 3] = ord(c);
+            mag = fmaxf(mag, fmaxf(fabsf(lo), fabsf(hi)));
+        }
+        word[4 * D] = ord(mag);
     }
-    atomicMax(&b->mag, ord(mag));
+#pragma unroll
+    for (int k = 0; k < kWords; k++) {
+        const uint32_t m = __reduce_max_sync(0xffffffffu, word[k]);
+        if (lane == 0) red[warp][k] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x < kWords) {
+        const int k = threadIdx.x, axis = k >> 2;
+        uint32_t m = red[0][k];
+        for (int w = 1; w < kT / 32; w++) m = max(m, red[w][k]);
+        if (k == 4 * D) atomicMax(&b->mag, m);
+        else if ((k & 3) == 0) atomicMin(&b->lo[axis], ~m);
+        else if ((k & 3) == 1) atomicMax(&b->hi[axis], m);
+        else if ((k & 3) == 2) atomicMin(&b->clo[axis], ~m);
+        else atomicMax(&b->chi[axis], m);
+    }
+    if (threadIdx.x == 0) {
+        if (s_bad) atomicOr(&b->bad, s_bad);
+        if (s_other) atomicAnd(&b->all_dirichlet, 0u);
+    }
 }
 
 __device__ __forceinline__ uint64_t spread21(uint64_t x) {  // 21 bits -> every third bit
@@ -136,23 +189,6 @@ __global__ void k_morton(uint32_t n, uint32_t n2, const float *__restrict__ box,
     val[i] = i;
 }
 
-__global__ void k_bitonic(uint32_t n2, uint32_t j, uint32_t k, uint64_t *key, uint32_t *val) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n2) return;
-    const uint32_t l = i ^ j;
-    if (l <= i) return;
-    const uint64_t ka = key[i], kb = key[l];
-    const uint32_t va = val[i], vb = val[l];
-    const bool greater = ka > kb || (ka == kb && va > vb);
-    const bool up = (i & k) == 0;
-    if (up == greater) {
-        key[i] = kb;
-        key[l] = ka;
-        val[i] = vb;
-        val[l] = va;
-    }
-}
-
 // common-prefix length of the augmented keys (code, index) at sorted positions a and b
 __device__ __forceinline__ int delta(const uint64_t *key, int64_t n, int64_t a, int64_t b) {
     if (b < 0 || b >= n) return -1;
@@ -162,6 +198,7 @@ __device__ __forceinline__ int delta(const uint64_t *key, int64_t n, int64_t a, 
 }
 
 constexpr uint32_t kLeafBit = 0x80000000u;
+constexpr uint32_t kNotWide = 0xFFFFFFFFu;
 
 // Binary radix tree: internal node i has children child[2i], child[2i+1] (kLeafBit | sorted
 // position for leaves) and covers sorted positions [first[i], last[i]].
@@ -200,16 +237,17 @@ __global__ void k_radix_tree(uint32_t n, const uint64_t *__restrict__ key, uint3
 
 // Boxes of the binary nodes, bottom-up: the second child to arrive at a parent writes its box.
 // A climb is bounded by the tree height (at most 96 levels for 64-bit codes plus 32 index bits);
-// a longer one can only come from a malformed tree and sets bit 5 of the error word.
-__global__ void k_boxes(uint32_t n, float pad, const uint32_t *__restrict__ val, const float *__restrict__ ebox,
+// a longer one can only come from a malformed tree and sets bit 6 of the error word.
+__global__ void k_boxes(uint32_t n, int dim, const uint32_t *__restrict__ val, const float *__restrict__ ebox,
                         const uint32_t *__restrict__ child, const uint32_t *__restrict__ parent_int,
-                        const uint32_t *__restrict__ parent_leaf, uint32_t *flags, float *ibox, uint32_t *err) {
+                        const uint32_t *__restrict__ parent_leaf, uint32_t *flags, float *ibox, Bounds *bd) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n || n < 2) return;
+    const float pad = box_pad(*bd, dim);
     uint32_t node = parent_leaf[s];
     for (int level = 0;; level++) {
         if (level > 128 || node >= n - 1) {
-            atomicOr(err, 32u);
+            atomicOr(&bd->bad, kBadTree);
             return;
         }
         __threadfence();
@@ -240,10 +278,6 @@ __global__ void k_boxes(uint32_t n, float pad, const uint32_t *__restrict__ val,
     }
 }
 
-struct Slot {
-    uint32_t code;  // binary child code (kLeafBit | sorted position, or internal index)
-};
-
 __device__ __forceinline__ uint32_t range_count(uint32_t code, const uint32_t *first, const uint32_t *last) {
     return (code & kLeafBit) ? 1u : last[code] - first[code] + 1u;
 }
@@ -264,93 +298,116 @@ __device__ __forceinline__ int wide_children(uint32_t b, const uint32_t *child, 
     return m;
 }
 
-// per frontier item: how many of its children become wide nodes
-__global__ void k_collapse_count(uint32_t cnt, const uint32_t *__restrict__ fb, const uint32_t *child,
-                                 const uint32_t *first, const uint32_t *last, uint32_t *ncount) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= cnt) return;
-    uint32_t ch[4];
-    const int m = wide_children(fb[t], child, first, last, ch);
-    uint32_t c = 0;
-    for (int k = 0; k < m; k++)
-        if (range_count(ch[k], first, last) > kLeafMax) c++;
-    ncount[t] = c;
+// Marks the binary nodes that become wide nodes (even depth, more than kLeafMax elements) and counts
+// them per block. A node's depth is its climb to the root: a level-by-level collapse needs a round
+// trip to the host per level (13 levels and 1.0 ms for 327,680 triangles; the climbs take 0.02 ms).
+__global__ void __launch_bounds__(kT) k_wide_mark(uint32_t n_int, const uint32_t *__restrict__ first,
+                                                  const uint32_t *__restrict__ last,
+                                                  const uint32_t *__restrict__ parent_int, uint32_t *__restrict__ rank,
+                                                  uint32_t *__restrict__ blk, Bounds *bd) {
+    __shared__ uint32_t warp_count[kT / 32];
+    const uint32_t i = blockIdx.x * kT + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    bool wide = false;
+    uint32_t depth = 0;
+    if (i < n_int && last[i] - first[i] + 1u > kLeafMax) {
+        uint32_t node = i;
+        while (node != 0u && depth <= 128u) {
+            node = parent_int[node];
+            depth++;
+        }
+        if (depth > 128u) atomicOr(&bd->bad, kBadTree);
+        wide = (depth & 1u) == 0u;
+    }
+    const uint32_t bits = __ballot_sync(0xffffffffu, wide);
+    const uint32_t deepest = __reduce_max_sync(0xffffffffu, wide ? depth / 2u + 1u : 0u);
+    if (lane == 0) {
+        warp_count[warp] = (uint32_t)__popc(bits);
+        if (deepest) atomicMax(&bd->depth, deepest);
+    }
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+    for (uint32_t w = 0; w < kT / 32; w++) {
+        if (w < warp) before += warp_count[w];
+        all += warp_count[w];
+    }
+    if (i < n_int) rank[i] = wide ? before + (uint32_t)__popc(bits & ((1u << lane) - 1u)) : kNotWide;
+    if (threadIdx.x == 0) blk[blockIdx.x] = all;
 }
 
 // exclusive scan of cnt values in one block; total written to *total
-__global__ void k_scan(uint32_t cnt, const uint32_t *__restrict__ in, uint32_t *out, uint32_t *total) {
+__global__ void __launch_bounds__(1024) k_scan(uint32_t cnt, uint32_t *v, uint32_t *total) {
     __shared__ uint32_t part[1024];
-    const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    const uint32_t chunk = (cnt + nt - 1) / nt;
-    const uint32_t b = tid * chunk, e = min(cnt, b + chunk);
+    const uint32_t tid = threadIdx.x;
+    const uint32_t chunk = (cnt + 1023u) / 1024u;
+    const uint32_t b = min(cnt, tid * chunk), e = min(cnt, b + chunk);
     uint32_t s = 0;
-    for (uint32_t i = b; i < e; i++) s += in[i];
+    for (uint32_t i = b; i < e; i++) s += v[i];
     part[tid] = s;
     __syncthreads();
-    if (tid == 0) {
-        uint32_t acc = 0;
-        for (uint32_t k = 0; k < nt; k++) {
-            const uint32_t v = part[k];
-            part[k] = acc;
-            acc += v;
-        }
-        *total = acc;
+    for (uint32_t o = 1; o < 1024u; o <<= 1) {
+        const uint32_t add = tid >= o ? part[tid - o] : 0u;
+        __syncthreads();
+        part[tid] += add;
+        __syncthreads();
     }
-    __syncthreads();
-    uint32_t acc = part[tid];
+    if (tid == 1023u) *total = part[1023];
+    uint32_t acc = part[tid] - s;
     for (uint32_t i = b; i < e; i++) {
-        out[i] = acc;
-        acc += in[i];
+        const uint32_t x = v[i];
+        v[i] = acc;
+        acc += x;
     }
 }
 
-// writes the wide node records of one frontier level and the next frontier
+// writes the wide node records
 template <int D>
-__global__ void k_collapse_write(uint32_t cnt, const uint32_t *__restrict__ fw, const uint32_t *__restrict__ fb,
-                                 const uint32_t *__restrict__ offs, uint32_t base, const uint32_t *child,
-                                 const uint32_t *first, const uint32_t *last, const uint32_t *__restrict__ val,
-                                 const float *__restrict__ ebox, const float *__restrict__ ibox, float pad, float *nodes,
-                                 uint32_t *nw, uint32_t *nb) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= cnt) return;
+__global__ void __launch_bounds__(kT) k_wide_write(uint32_t n_int, const uint32_t *__restrict__ rank,
+                                                   const uint32_t *__restrict__ blk,
+                                                   const uint32_t *__restrict__ child,
+                                                   const uint32_t *__restrict__ first,
+                                                   const uint32_t *__restrict__ last, const uint32_t *__restrict__ val,
+                                                   const float *__restrict__ ebox, const float *__restrict__ ibox,
+                                                   const Bounds *__restrict__ bd, float *__restrict__ nodes) {
+    const uint32_t t = blockIdx.x * kT + threadIdx.x;
+    if (t >= n_int || rank[t] == kNotWide) return;
+    const float pad = box_pad(*bd, D);
     constexpr int NF = D == 2 ? 24 : 32;
-    float *r = nodes + (size_t)fw[t] * NF;
+    float4 *r = reinterpret_cast<float4 *>(nodes + (size_t)(blk[blockIdx.x] + rank[t]) * NF);
     uint32_t ch[4];
-    const int m = wide_children(fb[t], child, first, last, ch);
-    uint32_t next = base + offs[t];
+    const int m = wide_children(t, child, first, last, ch);
+    float lo[D][4], hi[D][4];
+    uint32_t codes[4];
+#pragma unroll
     for (int k = 0; k < 4; k++) {
-        uint32_t code = kChildEmpty;
-        float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+        codes[k] = kChildEmpty;
+#pragma unroll
+        for (int a = 0; a < D; a++) lo[a][k] = hi[a][k] = 0.0f;
         if (k < m) {
             const uint32_t c = ch[k];
             const uint32_t count = range_count(c, first, last);
             const uint32_t f = (c & kLeafBit) ? (c & ~kLeafBit) : first[c];
-            if (count > kLeafMax) {
-                code = next;
-                nw[next - base] = next;
-                nb[next - base] = c;
-                next++;
-            } else {
-                code = 0x80000000u | ((count - 1u) << 28) | f;
-            }
+            codes[k] = count > kLeafMax ? blk[c / kT] + rank[c] : 0x80000000u | ((count - 1u) << 28) | f;
+            const uint32_t e = (c & kLeafBit) ? val[c & ~kLeafBit] : 0u;
+#pragma unroll
             for (int a = 0; a < D; a++) {
                 if (c & kLeafBit) {
-                    const uint32_t e = val[c & ~kLeafBit];
-                    lo[a] = ebox[(size_t)e * 9 + a] - pad;
-                    hi[a] = ebox[(size_t)e * 9 + 3 + a] + pad;
+                    lo[a][k] = ebox[(size_t)e * 9 + a] - pad;
+                    hi[a][k] = ebox[(size_t)e * 9 + 3 + a] + pad;
                 } else {
-                    lo[a] = ibox[(size_t)c * 6 + a];
-                    hi[a] = ibox[(size_t)c * 6 + 3 + a];
+                    lo[a][k] = ibox[(size_t)c * 6 + a];
+                    hi[a][k] = ibox[(size_t)c * 6 + 3 + a];
                 }
             }
         }
-        for (int a = 0; a < D; a++) {
-            r[4 * a + k] = lo[a];
-            r[4 * (D + a) + k] = hi[a];
-        }
-        r[4 * (2 * D) + k] = __uint_as_float(code);
-        r[4 * (2 * D + 1) + k] = 0.0f;  // padding to a 32-byte multiple
     }
+#pragma unroll
+    for (int a = 0; a < D; a++) {
+        r[a] = make_float4(lo[a][0], lo[a][1], lo[a][2], lo[a][3]);
+        r[D + a] = make_float4(hi[a][0], hi[a][1], hi[a][2], hi[a][3]);
+    }
+    r[2 * D] = make_float4(__uint_as_float(codes[0]), __uint_as_float(codes[1]), __uint_as_float(codes[2]),
+                           __uint_as_float(codes[3]));
+    r[2 * D + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // padding to a 32-byte multiple
 }
 
 // element records, intersection records, area and |g| weights in storage order (scene_build.cpp)
@@ -368,103 +425,58 @@ __global__ void k_records(uint32_t n, const uint32_t *__restrict__ val, const fl
     float al[3] = {0, 0, 0};
     if (alphas)
         for (int k = 0; k < D; k++) al[k] = alphas[(size_t)i * D + k];
+    float4 *r = reinterpret_cast<float4 *>(elems + (size_t)s * 16);
+    const float type = __int_as_float(types[i]);
     if constexpr (D == 2) {
-        float *r = elems + (size_t)s * 16;
         const float dx = v[2] - v[0], dy = v[3] - v[1];
         const float area = sqrtf(dx * dx + dy * dy);
-        r[0] = v[0]; r[1] = v[1]; r[2] = v[2]; r[3] = v[3];
-        r[4] = nn[0]; r[5] = nn[1]; r[6] = bv[0]; r[7] = bv[1];
-        r[8] = al[0]; r[9] = al[1]; r[10] = area; r[11] = __int_as_float(types[i]);
-        r[12] = 0.0f; r[13] = 0.0f; r[14] = 0.0f; r[15] = 0.0f;
+        r[0] = make_float4(v[0], v[1], v[2], v[3]);
+        r[1] = make_float4(nn[0], nn[1], bv[0], bv[1]);
+        r[2] = make_float4(al[0], al[1], area, type);
+        r[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         areas[s] = area;
         bvw[s] = area * (fabsf(bv[0]) + fabsf(bv[1])) / 2.0f;
     } else {
-        float *r = elems + (size_t)s * 16;
-        float *aux = elem_aux + (size_t)s * 4;
         const float u0 = v[6] - v[0], u1 = v[7] - v[1], u2 = v[8] - v[2];
         const float w0 = v[3] - v[0], w1 = v[4] - v[1], w2 = v[5] - v[2];
         const float x = u1 * w2 - u2 * w1;
         const float y = u2 * w0 - u0 * w2;
         const float z = u0 * w1 - u1 * w0;
         const float area = sqrtf(x * x + y * y + z * z) / 2.0f;
-        for (int k = 0; k < 9; k++) r[k] = v[k];
-        r[9] = nn[0]; r[10] = nn[1]; r[11] = nn[2];
-        r[12] = bv[0]; r[13] = bv[1]; r[14] = bv[2]; r[15] = __int_as_float(types[i]);
-        aux[0] = al[0]; aux[1] = al[1]; aux[2] = al[2]; aux[3] = area;
+        r[0] = make_float4(v[0], v[1], v[2], v[3]);
+        r[1] = make_float4(v[4], v[5], v[6], v[7]);
+        r[2] = make_float4(v[8], nn[0], nn[1], nn[2]);
+        r[3] = make_float4(bv[0], bv[1], bv[2], type);
+        reinterpret_cast<float4 *>(elem_aux)[s] = make_float4(al[0], al[1], al[2], area);
         areas[s] = area;
         bvw[s] = area * (fabsf(bv[0]) + fabsf(bv[1]) + fabsf(bv[2])) / 3.0f;
-        float *q = isect + (size_t)s * 16;
+        float4 *q = reinterpret_cast<float4 *>(isect + (size_t)s * 16);
         const float e1x = v[0] - v[3], e1y = v[1] - v[4], e1z = v[2] - v[5];
         const float e2x = v[0] - v[6], e2y = v[1] - v[7], e2z = v[2] - v[8];
-        q[0] = v[0]; q[1] = v[1]; q[2] = v[2];
-        q[3] = e1x; q[4] = e1y; q[5] = e1z;
-        q[6] = e2x; q[7] = e2y; q[8] = e2z;
-        q[9] = e1y * e2z - e1z * e2y;
-        q[10] = e1z * e2x - e1x * e2z;
-        q[11] = e1x * e2y - e1y * e2x;
-        q[12] = 0.0f; q[13] = 0.0f; q[14] = 0.0f; q[15] = 0.0f;
+        q[0] = make_float4(v[0], v[1], v[2], e1x);
+        q[1] = make_float4(e1y, e1z, e2x, e2y);
+        q[2] = make_float4(e2z, e1y * e2z - e1z * e2y, e1z * e2x - e1x * e2z, e1x * e2y - e1y * e2x);
+        q[3] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
 }
 
-// Kahan prefix sums, normalisation and the nondecreasing fix-up of scene_build.cpp's kahan_cdf:
-// thread 0 builds the area CDF, thread 1 the |g| CDF, each serially in storage order.
-__global__ void k_kahan_cdf(uint32_t n, const float *__restrict__ areas, const float *__restrict__ bvw,
-                            float *area_cdf, float *bv_cdf, float *totals) {
-    const int w = threadIdx.x;
-    if (w > 1) return;
-    const float *in = w == 0 ? areas : bvw;
-    float *cdf = w == 0 ? area_cdf : bv_cdf;
-    float sum = 0.0f, c = 0.0f;
-    for (uint32_t i = 0; i < n; i++) {
-        const float y = in[i] - c;
-        const float t = sum + y;
-        c = (t - sum) - y;
-        sum = t;
-        cdf[i] = sum;
-    }
-    const float total = sum;
-    totals[w] = total;
-    float prev = -INFINITY;
-    for (uint32_t i = 0; i < n; i++) {
-        float v = cdf[i] / total;
-        if (i > 0 && v < prev) v = prev;
-        cdf[i] = v;
-        prev = v;
-    }
-}
-
-// guide table (scene_build.cpp build_guide): first index whose CDF reaches (j - 1/2)/G
-__device__ __forceinline__ uint32_t guide_first(const float *cdf, uint32_t n, uint32_t G, uint32_t j) {
-    const double thr = ((double)j - 0.5) / (double)G;
-    uint32_t lo = 0, hi = n - 1;  // answer in [0, n-1]: first i with cdf[i] >= thr, else n-1
-    while (lo < hi) {
-        const uint32_t mid = lo + (hi - lo) / 2;
-        if ((double)cdf[mid] < thr) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
-}
-__global__ void k_guide(uint32_t n, uint32_t G, const float *__restrict__ cdf, uint32_t *rec) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= G) return;
-    const uint32_t lo = guide_first(cdf, n, G, j);
-    const uint32_t hi = (j + 2 < G) ? guide_first(cdf, n, G, j + 2) : n - 1;
-    rec[4 * (size_t)j + 0] = lo;
-    rec[4 * (size_t)j + 1] = hi;
-    rec[4 * (size_t)j + 2] = __float_as_uint(cdf[lo]);
-    rec[4 * (size_t)j + 3] = __float_as_uint(cdf[min(lo + 1, n - 1)]);
-}
-
+// The build's scratch, one allocation: take() first adds up the sizes, after allocate() it hands out
+// the pointers in the same order.
 struct Tmp {
-    std::vector<void *> ptrs;
+    char *base = nullptr;
+    size_t used = 0;
     ~Tmp() {
-        for (void *p : ptrs) cudaFree(p);
+        if (base) cudaFree(base);
     }
-    template <class T> cudaError_t alloc(T **p, size_t count) {
+    template <class T> void take(T **p, size_t count) {
+        *p = base ? (T *)(base + used) : nullptr;
+        used += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
+    }
+    cudaError_t allocate() {
         void *q = nullptr;
-        cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-        if (e == cudaSuccess) ptrs.push_back(q);
-        *p = (T *)q;
+        const cudaError_t e = cudaMalloc(&q, used);
+        if (e == cudaSuccess) base = (char *)q;
+        used = 0;
         return e;
     }
 };
@@ -479,10 +491,29 @@ std::string build_impl(uint32_t n, const float *verts, const float *normals, con
     do {                                     \
         if ((ce = (x)) != cudaSuccess) return "CUDA error"; \
     } while (0)
-    float *box = nullptr;
-    Bounds *bd = nullptr;
-    WOB_CK(tmp.alloc(&box, (size_t)n * 9));
-    WOB_CK(tmp.alloc(&bd, 1));
+    const uint32_t n2 = sort_padded(n), n_int = n > 1 ? n - 1 : 1;
+    float *box, *ibox, *areas, *bvw;
+    Bounds *bd;
+    uint64_t *key;
+    uint32_t *val, *child, *first, *last, *pint, *pleaf, *flags, *blk;
+    unsigned char *kahan;
+    auto lay_out = [&]() {
+        tmp.take(&key, n2);
+        tmp.take(&bd, 1);
+        tmp.take(&kahan, kahan_scratch_bytes(n, 2));
+        tmp.take(&val, n2);
+        tmp.take(&box, (size_t)n * 9);
+        tmp.take(&areas, n);
+        tmp.take(&bvw, n);
+        tmp.take(&child, 2 * (size_t)n_int);
+        for (uint32_t **p : {&first, &last, &pint, &flags}) tmp.take(p, n_int);
+        tmp.take(&pleaf, n);
+        tmp.take(&ibox, 6 * (size_t)n_int);
+        tmp.take(&blk, n_int / kT + 1);
+    };
+    lay_out();  // measures; after the allocation the same calls hand out the pointers
+    WOB_CK(tmp.allocate());
+    lay_out();
     Bounds init;
     for (int k = 0; k < 3; k++) {
         init.lo[k] = init.clo[k] = 0xFFFFFFFFu;
@@ -491,49 +522,31 @@ std::string build_impl(uint32_t n, const float *verts, const float *normals, con
     init.mag = 0u;
     init.bad = 0u;
     init.all_dirichlet = 1u;
+    init.n_nodes = init.depth = 0u;
+    init.totals[0] = init.totals[1] = 0.0f;
     WOB_CK(cudaMemcpyAsync(bd, &init, sizeof(Bounds), cudaMemcpyHostToDevice, st));
     k_validate<D><<<blocks(n), kT, 0, st>>>(n, verts, normals, bvals, alphas, types, box, bd);
     WOB_CK(cudaGetLastError());
-    Bounds hb;
-    WOB_CK(cudaMemcpyAsync(&hb, bd, sizeof(Bounds), cudaMemcpyDeviceToHost, st));
-    WOB_CK(cudaStreamSynchronize(st));
-    if (hb.bad & 1u) return "vertices must be finite";
-    if (hb.bad & 2u) return "normals must be finite";
-    if (hb.bad & 4u) return "boundary values must be finite";
-    if (hb.bad & 8u) return "robin alphas must be finite";
-    if (hb.bad & 16u) return "boundary_types must be 0 (Dirichlet), 1 (Neumann) or 2 (Robin)";
-    if (hb.bad & 32u) return "normals must be unit vectors";
-    out.all_dirichlet = hb.all_dirichlet != 0u;
-    // padding of the host build: 1e-5 (extent + max |coordinate|)
-    float ext = 0.0f;
-    for (int k = 0; k < D; k++) ext = std::max(ext, unord(hb.hi[k]) - unord(hb.lo[k]));
-    const float pad = 1e-5f * (ext + unord(hb.mag)) + 1e-30f;
 
     // Morton codes and the sort
-    uint32_t n2 = 1;
-    while (n2 < n) n2 <<= 1;
-    uint64_t *key = nullptr;
-    uint32_t *val = nullptr;
-    WOB_CK(tmp.alloc(&key, n2));
-    WOB_CK(tmp.alloc(&val, n2));
     k_morton<D><<<blocks(n2), kT, 0, st>>>(n, n2, box, bd, key, val);
-    for (uint32_t k = 2; k <= n2; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) k_bitonic<<<blocks(n2), kT, 0, st>>>(n2, j, k, key, val);
     WOB_CK(cudaGetLastError());
+    WOB_CK(launch_sort_keys(n2, key, val, st));
 
     constexpr int NF = D == 2 ? 24 : 32;
-    const uint32_t n_int = n > 1 ? n - 1 : 1;
     float *nodes = nullptr;
     WOB_CK(cudaMalloc(&nodes, (size_t)n_int * NF * 4));
     out.nodes = nodes;
     out.nodes_bytes = (size_t)n_int * NF * 4;
-    uint32_t n_nodes = 1, depth = 1;
     if (n <= kLeafMax) {
         // one wide node holding one leaf (scene_build.cpp)
         std::vector<float> root(NF, 0.0f);
         std::vector<float> hbox(9 * (size_t)n);
+        Bounds hb;
         WOB_CK(cudaMemcpyAsync(hbox.data(), box, hbox.size() * 4, cudaMemcpyDeviceToHost, st));
+        WOB_CK(cudaMemcpyAsync(&hb, bd, sizeof(Bounds), cudaMemcpyDeviceToHost, st));
         WOB_CK(cudaStreamSynchronize(st));
+        const float pad = box_pad(hb, D);
         for (int a = 0; a < D; a++) {
             float lo = INFINITY, hi = -INFINITY;
             for (uint32_t i = 0; i < n; i++) {
@@ -546,58 +559,21 @@ std::string build_impl(uint32_t n, const float *verts, const float *normals, con
         const uint32_t codes[4] = {make_leaf(0, n), kChildEmpty, kChildEmpty, kChildEmpty};
         for (int k = 0; k < 4; k++) std::memcpy(&root[4 * (2 * D) + k], &codes[k], 4);
         WOB_CK(cudaMemcpyAsync(nodes, root.data(), NF * 4, cudaMemcpyHostToDevice, st));
+        WOB_CK(cudaStreamSynchronize(st));
     } else {
-        uint32_t *child, *first, *last, *pint, *pleaf, *flags;
-        float *ibox;
-        WOB_CK(tmp.alloc(&child, 2 * (size_t)n_int));
-        WOB_CK(tmp.alloc(&first, n_int));
-        WOB_CK(tmp.alloc(&last, n_int));
-        WOB_CK(tmp.alloc(&pint, n_int));
-        WOB_CK(tmp.alloc(&pleaf, n));
-        WOB_CK(tmp.alloc(&flags, n_int));
-        WOB_CK(tmp.alloc(&ibox, 6 * (size_t)n_int));
         WOB_CK(cudaMemsetAsync(flags, 0, (size_t)n_int * 4, st));
         k_radix_tree<<<blocks(n - 1), kT, 0, st>>>(n, key, child, first, last, pint, pleaf);
-        k_boxes<<<blocks(n), kT, 0, st>>>(n, pad, val, box, child, pint, pleaf, flags, ibox, &bd->bad);
+        k_boxes<<<blocks(n), kT, 0, st>>>(n, D, val, box, child, pint, pleaf, flags, ibox, bd);
+        uint32_t *rank = flags;  // the boxes' arrival counts are done with
+        k_wide_mark<<<blocks(n_int), kT, 0, st>>>(n_int, first, last, pint, rank, blk, bd);
+        k_scan<<<1, 1024, 0, st>>>(blocks(n_int), blk, &bd->n_nodes);
+        k_wide_write<D><<<blocks(n_int), kT, 0, st>>>(n_int, rank, blk, child, first, last, val, box, ibox, bd, nodes);
         WOB_CK(cudaGetLastError());
-        // top-down collapse, one level per step
-        uint32_t *fw[2], *fb[2], *cnt, *offs, *total;
-        for (int b = 0; b < 2; b++) {
-            WOB_CK(tmp.alloc(&fw[b], n_int));
-            WOB_CK(tmp.alloc(&fb[b], n_int));
-        }
-        WOB_CK(tmp.alloc(&cnt, n_int));
-        WOB_CK(tmp.alloc(&offs, n_int));
-        WOB_CK(tmp.alloc(&total, 1));
-        const uint32_t zero = 0;
-        WOB_CK(cudaMemcpyAsync(fw[0], &zero, 4, cudaMemcpyHostToDevice, st));
-        WOB_CK(cudaMemcpyAsync(fb[0], &zero, 4, cudaMemcpyHostToDevice, st));
-        uint32_t level_count = 1, cur = 0;
-        depth = 0;
-        while (level_count > 0) {
-            depth++;
-            if (3 * depth + 2 > kTraversalStack) return "BVH too deep for the traversal stack";
-            k_collapse_count<<<blocks(level_count), kT, 0, st>>>(level_count, fb[cur], child, first, last, cnt);
-            k_scan<<<1, 1024, 0, st>>>(level_count, cnt, offs, total);
-            k_collapse_write<D><<<blocks(level_count), kT, 0, st>>>(level_count, fw[cur], fb[cur], offs, n_nodes,
-                                                                   child, first, last, val, box, ibox, pad, nodes,
-                                                                   fw[1 - cur], fb[1 - cur]);
-            WOB_CK(cudaGetLastError());
-            uint32_t next = 0;
-            WOB_CK(cudaMemcpyAsync(&next, total, 4, cudaMemcpyDeviceToHost, st));
-            WOB_CK(cudaStreamSynchronize(st));
-            n_nodes += next;
-            level_count = next;
-            cur = 1 - cur;
-        }
     }
-    out.n_nodes = n_nodes;
-    out.depth = depth;
 
     // records, CDFs, guides
     const int EF = 16;
-    float *elems = nullptr, *elem_aux = nullptr, *isect = nullptr, *area_cdf = nullptr, *bv_cdf = nullptr, *areas,
-          *bvw, *totals;
+    float *elems = nullptr, *elem_aux = nullptr, *isect = nullptr, *area_cdf = nullptr, *bv_cdf = nullptr;
     WOB_CK(cudaMalloc(&elems, (size_t)n * EF * 4));
     out.elems = elems;
     out.elems_bytes = (size_t)n * EF * 4;
@@ -615,22 +591,29 @@ std::string build_impl(uint32_t n, const float *verts, const float *normals, con
     WOB_CK(cudaMalloc(&bv_cdf, (size_t)n * 4));
     out.bv_cdf = bv_cdf;
     out.bv_cdf_bytes = (size_t)n * 4;
-    WOB_CK(tmp.alloc(&areas, n));
-    WOB_CK(tmp.alloc(&bvw, n));
-    WOB_CK(tmp.alloc(&totals, 2));
     k_records<D><<<blocks(n), kT, 0, st>>>(n, val, verts, normals, bvals, alphas, types, elems, elem_aux, isect, areas,
                                            bvw);
-    k_kahan_cdf<<<1, 32, 0, st>>>(n, areas, bvw, area_cdf, bv_cdf, totals);
-    WOB_CK(cudaGetLastError());
-    float ht[2];
-    WOB_CK(cudaMemcpyAsync(ht, totals, 8, cudaMemcpyDeviceToHost, st));
+    const float *weights[2] = {areas, bvw};
+    float *cdfs[2] = {area_cdf, bv_cdf};
+    WOB_CK(launch_kahan_cdf(n, 2, weights, cdfs, bd->totals, kahan, st));
+    Bounds hb;
     WOB_CK(cudaMemcpyAsync(&hb, bd, sizeof(Bounds), cudaMemcpyDeviceToHost, st));
     out.order.resize(n);
     WOB_CK(cudaMemcpyAsync(out.order.data(), val, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
     WOB_CK(cudaStreamSynchronize(st));
-    if (hb.bad & 32u) return "BVH build failed: malformed radix tree";
-    out.total_area = ht[0];
-    out.total_bv = ht[1];
+    if (hb.bad & 1u) return "vertices must be finite";
+    if (hb.bad & 2u) return "normals must be finite";
+    if (hb.bad & 4u) return "boundary values must be finite";
+    if (hb.bad & 8u) return "robin alphas must be finite";
+    if (hb.bad & 16u) return "boundary_types must be 0 (Dirichlet), 1 (Neumann) or 2 (Robin)";
+    if (hb.bad & 32u) return "normals must be unit vectors";
+    if (hb.bad & kBadTree) return "BVH build failed: malformed radix tree";
+    out.all_dirichlet = hb.all_dirichlet != 0u;
+    out.n_nodes = n <= kLeafMax ? 1u : hb.n_nodes;
+    out.depth = n <= kLeafMax ? 1u : hb.depth;
+    if (3 * out.depth + 2 > kTraversalStack) return "BVH too deep for the traversal stack";
+    out.total_area = hb.totals[0];
+    out.total_bv = hb.totals[1];
     if (!(out.total_area > 0.0f) || !std::isfinite(out.total_area)) return "total boundary area must be positive and finite";
     const uint32_t G = std::max<uint32_t>(1u, std::min<uint32_t>(n, 1u << 22));
     uint32_t *ag = nullptr, *bg = nullptr;
@@ -638,16 +621,15 @@ std::string build_impl(uint32_t n, const float *verts, const float *normals, con
     out.area_guide = ag;
     out.area_guide_bytes = (size_t)G * 16;
     out.area_G = G;
-    k_guide<<<blocks(G), kT, 0, st>>>(n, G, area_cdf, ag);
+    WOB_CK(launch_guide(n, G, area_cdf, ag, st));
     out.bv_valid = out.total_bv > 0.0f && std::isfinite(out.total_bv);
     const uint32_t Gb = out.bv_valid ? G : 1u;
     WOB_CK(cudaMalloc(&bg, (size_t)Gb * 16));
     out.bv_guide = bg;
     out.bv_guide_bytes = (size_t)Gb * 16;
     out.bv_G = Gb;
-    if (out.bv_valid) k_guide<<<blocks(G), kT, 0, st>>>(n, G, bv_cdf, bg);
+    if (out.bv_valid) WOB_CK(launch_guide(n, G, bv_cdf, bg, st));
     else WOB_CK(cudaMemsetAsync(bg, 0, 16, st));
-    WOB_CK(cudaGetLastError());
     WOB_CK(cudaStreamSynchronize(st));
 #undef WOB_CK
     return "";
