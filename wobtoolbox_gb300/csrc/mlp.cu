@@ -13,6 +13,7 @@
 #include "mlp_train.hpp"
 
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -157,6 +158,119 @@ __global__ void fourier_kernel(const float *__restrict__ in, const float *__rest
         sincospi_own(2.0f * t, &s, &c);
         phi[(long)i * (2 * n_freq) + f] = s;
         phi[(long)i * (2 * n_freq) + n_freq + f] = c;
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// Inference in one kernel: a warp carries 16 rows through the whole network in registers. The m16n8
+// accumulators of a layer are, packed to BF16 in pairs, the m16n8k16 A fragments of the next one, and
+// the Fourier features are computed in that layout (a lane's sine and cosine columns belong to the
+// same frequencies), so the activations touch no memory; the weights stay in shared memory as BF16,
+// rows padded to 72 values (a fragment load touches 32 banks). The products, their order over k and
+// every rounding are those of the layer-by-layer kernels above (gemm_bf16_kernel), so the outputs
+// have the same bits. 327,680 rows: 0.81 ms layer by layer (FP32 pre-activations and activations
+// through HBM), 0.145 ms here, bound by issuing the SiLUs (an exponential and a division each, 256 a
+// row); mma.sync rather than tcgen05 because the products are a twentieth of that issue.
+// ------------------------------------------------------------------------------------------
+constexpr int kInferWarps = 8;
+constexpr int kWPad = kWidth + 8;  // BF16 values per weight row in shared memory
+
+struct InferArgs {
+    const float *params, *freqs, *in;
+    float *out;
+    uint32_t n, hidden, out_dim;
+};
+
+__host__ __device__ constexpr size_t infer_smem(uint32_t hidden) {
+    return (size_t)(hidden + 1) * kWidth * (kWPad * 2 + 4) + 32 * kFeatIn * 4;
+}
+
+__global__ void __launch_bounds__(32 * kInferWarps) infer_kernel(InferArgs g) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int layers = (int)g.hidden + 1, out_dim = (int)g.out_dim;
+    __nv_bfloat16 *W = reinterpret_cast<__nv_bfloat16 *>(smem_raw);  // [layer][out][kWPad]
+    float *bias = reinterpret_cast<float *>(W + (size_t)layers * kWidth * kWPad);  // [layer][64]
+    float *fr = bias + layers * kWidth;                                            // [32][6]
+    for (int i = threadIdx.x; i < layers * kWidth * kWidth; i += blockDim.x) {
+        const int l = i / (kWidth * kWidth), o = i / kWidth % kWidth, k = i % kWidth;
+        const float *p = g.params + (size_t)l * (kWidth * kWidth + kWidth);
+        W[(l * kWidth + o) * kWPad + k] = __float2bfloat16_rn(l + 1 < layers || o < out_dim ? p[o * kWidth + k] : 0.0f);
+    }
+    for (int i = threadIdx.x; i < layers * kWidth; i += blockDim.x) {
+        const int l = i / kWidth, o = i % kWidth, fo = l + 1 < layers ? kWidth : out_dim;
+        bias[i] = o < fo ? g.params[(size_t)l * (kWidth * kWidth + kWidth) + (size_t)fo * kWidth + o] : 0.0f;
+    }
+    for (int i = threadIdx.x; i < 32 * kFeatIn; i += blockDim.x) fr[i] = g.freqs[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+    const uint32_t tiles = (g.n + 15u) / 16u;
+    for (uint32_t t = blockIdx.x * kInferWarps + (threadIdx.x >> 5); t < tiles; t += gridDim.x * kInferWarps) {
+        uint32_t a[4][4];
+        {
+            float v[2][kFeatIn];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const uint32_t row = t * 16u + gid + 8 * h;
+#pragma unroll
+                for (int k = 0; k < kFeatIn; k++) v[h][k] = row < g.n ? g.in[(size_t)row * kFeatIn + k] : 0.0f;
+            }
+#pragma unroll
+            for (int kk = 0; kk < 2; kk++)
+#pragma unroll
+                for (int c = 0; c < 2; c++) {  // columns 16 kk + 8 c + 2 tig and + 1
+                    float sn[2][2], cs[2][2];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const float *b = fr + (16 * kk + 8 * c + 2 * tig + e) * kFeatIn;
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            float x = 0.0f;
+#pragma unroll
+                            for (int k = 0; k < kFeatIn; k++) x = x + b[k] * v[h][k];
+                            sincospi_own(2.0f * x, &sn[h][e], &cs[h][e]);
+                        }
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        a[kk][2 * c + h] = pack_bf16(sn[h][0], sn[h][1]);
+                        a[kk + 2][2 * c + h] = pack_bf16(cs[h][0], cs[h][1]);
+                    }
+                }
+        }
+        for (int l = 0; l < layers; l++) {
+            const bool last = l + 1 == layers;
+            const uint32_t *Wl = reinterpret_cast<const uint32_t *>(W + (size_t)l * kWidth * kWPad);
+            uint32_t next[4][4];
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                if (last && j * 8 >= out_dim) break;
+                float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                const uint32_t *w = Wl + (j * 8 + gid) * (kWPad / 2) + tig;
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++) {
+                    const uint32_t b[2] = {w[8 * kk], w[8 * kk + 4]};
+                    mma_bf16_16816(acc, a[kk], b);
+                }
+                const float b0 = bias[l * kWidth + j * 8 + 2 * tig], b1 = bias[l * kWidth + j * 8 + 2 * tig + 1];
+                if (last) {
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const uint32_t row = t * 16u + gid + (r >= 2 ? 8 : 0);
+                        const int col = j * 8 + 2 * tig + (r & 1);
+                        if (row < g.n && col < out_dim) g.out[(size_t)row * out_dim + col] = acc[r] + (r & 1 ? b1 : b0);
+                    }
+                } else {
+                    next[j >> 1][2 * (j & 1)] = pack_bf16(silu(acc[0] + b0), silu(acc[1] + b1));
+                    next[j >> 1][2 * (j & 1) + 1] = pack_bf16(silu(acc[2] + b0), silu(acc[3] + b1));
+                }
+            }
+            if (!last) {
+#pragma unroll
+                for (int kk = 0; kk < 4; kk++)
+#pragma unroll
+                    for (int r = 0; r < 4; r++) a[kk][r] = next[kk][r];
+            }
+        }
     }
 }
 
@@ -521,13 +635,23 @@ int wob_mlp_set_params(wob_mlp m, const float *params) {
 int wob_mlp_forward(wob_mlp m, const float *inputs, uint32_t n, float *outputs, void *stream) {
     if (!m || (!inputs && n) || (!outputs && n)) return mfail(WOB_ERR_INVALID_ARGUMENT, "mlp, inputs and outputs are required");
     if (n == 0) return WOB_OK;
-    std::lock_guard<std::mutex> lock(m->mu);
-    cudaStream_t st = (cudaStream_t)stream;
-    cudaError_t e = m->ensure(n);
-    if (e != cudaSuccess) return mfail_cuda(e, "MLP workspace");
-    if ((e = forward_impl(m, inputs, n, st)) != cudaSuccess) return mfail_cuda(e, "MLP forward");
-    e = cudaMemcpyAsync(outputs, m->Y, (size_t)n * m->out_dim * 4, cudaMemcpyDeviceToDevice, st);
-    return e == cudaSuccess ? WOB_OK : mfail_cuda(e, "MLP forward copy");
+    using namespace wobgb;
+    const InferArgs a{m->params, m->freqs, inputs, outputs, n, m->hidden, m->out_dim};
+    const size_t smem = infer_smem(m->hidden);
+    cudaError_t e = cudaSuccess;
+    if (smem > 48u * 1024u &&
+        (e = cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        return mfail_cuda(e, "MLP forward");
+    int dev = 0, sms = 0, per_sm = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, infer_kernel, 32 * kInferWarps, smem)) != cudaSuccess)
+        return mfail_cuda(e, "MLP forward");
+    const uint32_t need = ((n + 15u) / 16u + kInferWarps - 1u) / kInferWarps;
+    const uint32_t grid = std::min(need, (uint32_t)(sms * std::max(per_sm, 1)));
+    infer_kernel<<<grid, 32 * kInferWarps, smem, (cudaStream_t)stream>>>(a);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? WOB_OK : mfail_cuda(e, "MLP forward");
 }
 
 int wob_mlp_gradient(wob_mlp m, const float *inputs, const float *targets, uint32_t n, float *grad, float *loss,
