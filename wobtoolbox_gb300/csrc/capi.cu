@@ -15,6 +15,7 @@
 #include "walk_generic.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -348,6 +349,8 @@ static int scene_create_impl(int dim, uint32_t n_elems, const float *vertices, c
         s->release_all();
         return fail_cuda(e, "uploading the scene");
     }
+    s->host.release_tables();
+    s->host.host_built = true;
     *out = owner.release();
     return WOB_OK;
 }
@@ -937,20 +940,15 @@ int scene_clone_impl(wob_scene src, wob_scene *out) {
     std::unique_ptr<wob_scene_s> owner(new wob_scene_s());
     wob_scene_s *s = owner.get();
     s->device = src->device;
-    // host copy: what wob_scene_add_boundary_offsets and a further clone read (the element records,
-    // areas, storage order, |g| tables and scalars); the BVH, intersection records, area tables and
-    // line grid stay on the device only, shared with the source
+    // the host keeps the storage order and scalars; records and tables live on the device only
     const wobgb::HostScene &h0 = src->host;
     wobgb::HostScene &h = s->host;
     h.dim = h0.dim;
     h.n = h0.n;
     h.order = h0.order;
-    h.elems = h0.elems;
-    h.elem_aux = h0.elem_aux;
+    h.host_built = h0.host_built;
     h.alpha_const = h0.alpha_const;
     h.alpha_value = h0.alpha_value;
-    h.bv_cdf = h0.bv_cdf;
-    h.bv_guide = h0.bv_guide;
     h.total_area = h0.total_area;
     h.total_bv = h0.total_bv;
     h.bv_valid = h0.bv_valid;
@@ -994,46 +992,63 @@ int scene_clone_impl(wob_scene src, wob_scene *out) {
 int scene_add_boundary_offsets_impl(wob_scene s, const float *delta, uint32_t n, int on_device, void *stream) {
     if (!s || !delta) return fail(WOB_ERR_INVALID_ARGUMENT, "scene and delta are required");
     if (n != s->host.n) return fail(WOB_ERR_INVALID_ARGUMENT, "need one offset per element");
-    if (s->host.elems.empty()) return fail(WOB_ERR_UNSUPPORTED, "the scene keeps no host records (built on the device)");
+    if (!s->host.host_built) return fail(WOB_ERR_UNSUPPORTED, "the scene keeps no host records (built on the device)");
     DeviceGuard g(s->device);
     cudaStream_t st = (cudaStream_t)stream;
-    std::vector<float> d(n);
-    cudaError_t e;
-    if (on_device) {
-        if ((e = cudaMemcpyAsync(d.data(), delta, (size_t)n * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(st)) != cudaSuccess)
-            return fail_cuda(e, "reading the offsets");
-    } else {
-        std::memcpy(d.data(), delta, (size_t)n * 4);
-    }
-    for (uint32_t i = 0; i < n; i++)
-        if (!(d[i] == d[i]) || d[i] > 3.0e38f || d[i] < -3.0e38f)
-            return fail(WOB_ERR_INVALID_ARGUMENT, "offsets must be finite");
+    // everything on the device: the records' adds and the new |g| tables, in buffers that replace the
+    // scene's once the offsets are known to be finite (a clone's source keeps the shared old ones)
+    DevBuf scratch, cdf, guide;
     wobgb::HostScene &h = s->host;
-    const int EF = wobgb::elem_record_floats(h.dim);
-    const int first = h.dim == 2 ? 6 : 12;
-    for (uint32_t i = 0; i < n; i++)
-        for (int k = 0; k < h.dim; k++) h.elems[(size_t)i * EF + first + k] = h.elems[(size_t)i * EF + first + k] + d[i];
-    // the device records get the same adds (offsets read from the caller's device buffer, or from
-    // a scratch copy of the host array)
-    DevBuf scratch;
+    const uint32_t G = std::min<uint32_t>(n, 1u << 22);
+    const size_t work = wobgb::offset_scratch_bytes(n);
+    auto alloc = [](DevBuf &b, size_t bytes) {
+        const cudaError_t r = cudaMalloc(&b.ptr, bytes);
+        if (r == cudaSuccess) b.bytes = bytes;
+        return r;
+    };
+    auto drop = [&] {
+        for (DevBuf *b : {&scratch, &cdf, &guide}) b->release();
+    };
+    wobgb::OffsetResult res{};
     const float *dd = delta;
-    if (!on_device) {
-        if ((e = upload(scratch, d.data(), (size_t)n * 4)) != cudaSuccess) return fail_cuda(e, "uploading the offsets");
-        dd = (const float *)scratch.ptr;
+    cudaError_t e;
+    if ((e = alloc(scratch, work + (on_device ? 0 : (size_t)n * 4))) != cudaSuccess ||
+        (e = alloc(cdf, (size_t)n * 4)) != cudaSuccess || (e = alloc(guide, (size_t)G * 16)) != cudaSuccess) {
+        drop();
+        return fail_cuda(e, "allocating the boundary value tables");
     }
-    e = wobgb::launch_add_boundary_offsets((float *)s->elems.ptr, dd, n, (uint32_t)EF, (uint32_t)first,
-                                           (uint32_t)h.dim, st);
-    wobgb::rebuild_bv_tables(h);
-    s->bv_G = (uint32_t)(h.bv_guide.size() / 4);
-    if (e != cudaSuccess || (e = cudaStreamSynchronize(st)) != cudaSuccess ||
-        (e = upload(s->bv_cdf, h.bv_cdf.data(), h.bv_cdf.size() * 4)) != cudaSuccess ||
-        (e = upload(s->bv_guide, h.bv_guide.data(), h.bv_guide.size() * 4)) != cudaSuccess) {
-        scratch.release();
+    if (!on_device) {
+        dd = (const float *)((char *)scratch.ptr + work);
+        e = cudaMemcpyAsync((void *)dd, delta, (size_t)n * 4, cudaMemcpyHostToDevice, st);
+    }
+    if (e != cudaSuccess ||
+        (e = wobgb::launch_boundary_offsets(h.dim, n, dd, (float *)s->elems.ptr, (const float4 *)s->elem_aux.ptr,
+                                            (float *)cdf.ptr, G, (uint32_t *)guide.ptr, scratch.ptr, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&res, scratch.ptr, sizeof res, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess) {
+        drop();
         return fail_cuda(e, "updating the boundary values");
     }
+    if (res.bad) {
+        drop();
+        return fail(WOB_ERR_INVALID_ARGUMENT, "offsets must be finite");
+    }
+    h.total_bv = res.total;
+    h.bv_valid = res.total > 0.0f && std::isfinite(res.total);
+    s->bv_cdf.release();
+    s->bv_guide.release();
+    s->bv_cdf = cdf;
+    if (h.bv_valid) {
+        s->bv_guide = guide;
+        s->bv_G = G;
+    } else {  // no |g| sampling: one empty guide record
+        const uint32_t none[4] = {0u, 0u, 0u, 0u};
+        guide.release();
+        s->bv_G = 1u;
+        e = upload(s->bv_guide, none, sizeof none);
+    }
     scratch.release();
-    return WOB_OK;
+    return e == cudaSuccess ? WOB_OK : fail_cuda(e, "updating the boundary values");
 }
 
 // Triangle sources and clusters of sigma~ in a scratch allocation freed on return.

@@ -40,6 +40,7 @@
 // This unit is compiled with FMA contraction (it is not part of the bit-exact walk).
 #include "device_common.cuh"
 #include "launch.hpp"
+#include "sort_keys.hpp"
 
 namespace wobgb {
 
@@ -162,7 +163,7 @@ __device__ __forceinline__ float warp_max_f(float v) {
 }
 
 // Morton order of evaluation points: bounds (order-preserving integer atomics), 30-bit codes (10
-// bits a coordinate), a bitonic sort of {code, index} keys padded to a power of two.
+// bits a coordinate), a sort of {code, index} keys padded to a power of two (k_sort.cu).
 __device__ __forceinline__ uint32_t ordered_bits(float f) {
     const uint32_t u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
@@ -183,11 +184,13 @@ __global__ void bounds_init_kernel(uint32_t *bb) {
 }
 __global__ void pts_bounds_kernel(const float *__restrict__ pts, uint32_t n, uint32_t *__restrict__ bb) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     for (int k = 0; k < 3; k++) {
-        const uint32_t o = ordered_bits(pts[(size_t)i * 3 + k]);
-        atomicMin(bb + k, o);
-        atomicMax(bb + 3 + k, o);
+        const uint32_t o = i < n ? ordered_bits(pts[(size_t)i * 3 + k]) : 0u;
+        const uint32_t lo = __reduce_min_sync(0xffffffffu, i < n ? o : 0xffffffffu), hi = __reduce_max_sync(0xffffffffu, o);
+        if ((threadIdx.x & 31u) == 0) {
+            atomicMin(bb + k, lo);
+            atomicMax(bb + 3 + k, hi);
+        }
     }
 }
 __global__ void pts_morton_kernel(const float *__restrict__ pts, uint32_t n, uint32_t n2, const uint32_t *__restrict__ bb,
@@ -207,18 +210,6 @@ __global__ void pts_morton_kernel(const float *__restrict__ pts, uint32_t n, uin
     }
     key[i] = ((uint64_t)code << 32) | i;
 }
-__global__ void bitonic_kernel(uint32_t n2, uint32_t j, uint32_t k, uint64_t *__restrict__ key) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n2) return;
-    const uint32_t l = i ^ j;
-    if (l <= i) return;
-    const uint64_t a = key[i], b = key[l];
-    if (((i & k) == 0) == (a > b)) {
-        key[i] = b;
-        key[l] = a;
-    }
-}
-
 // One warp per cluster: the record {z, r_far}, {M0, M1}, {M2xx, M2yy, M2zz, M2xy}, {M2xz, M2yz,
 // trace M2, 0}; r_far = max(rho / theta, rho + eta), infinite for theta = 0.
 __global__ void cv_cluster_kernel(uint32_t n, const float4 *__restrict__ src, const float *__restrict__ near2,
@@ -529,25 +520,7 @@ __global__ void element_frames_kernel(SceneView<D> s, float *__restrict__ out) {
     }
 }
 
-// Record i's vertex boundary values (record floats [first, first + dim)) plus delta[i]: the same
-// single-precision add as the host copy's update, so the two copies stay identical.
-__global__ void add_boundary_offsets_kernel(float *__restrict__ elems, const float *__restrict__ delta, uint32_t n,
-                                            uint32_t record_floats, uint32_t first, uint32_t dim) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float d = delta[i];
-    float *r = elems + (size_t)i * record_floats + first;
-    for (uint32_t k = 0; k < dim; k++) r[k] = r[k] + d;
-}
-
 }  // namespace
-
-cudaError_t launch_add_boundary_offsets(float *elems, const float *delta, uint32_t n, uint32_t record_floats,
-                                        uint32_t first, uint32_t dim, cudaStream_t stream) {
-    if (n == 0) return cudaSuccess;
-    add_boundary_offsets_kernel<<<(n + 255) / 256, 256, 0, stream>>>(elems, delta, n, record_floats, first, dim);
-    return cudaGetLastError();
-}
 
 template <int D> cudaError_t launch_element_frames(const SceneView<D> &s, float *out, cudaStream_t stream) {
     element_frames_kernel<D><<<(s.n_elems + 255) / 256, 256, 0, stream>>>(s, out);
@@ -581,8 +554,7 @@ cudaError_t launch_cv_residual(const SceneView<3> &s, const float4 *src, const f
 }
 
 uint32_t cv_point_order_words(uint32_t n_points) {
-    uint32_t n2 = 1;
-    while (n2 < n_points) n2 <<= 1;
+    const uint32_t n2 = sort_padded(n_points);
     // n2 keys of 8 bytes, the 6 bound words (padded to 8), the parts' FP64 sums
     return 2 * n2 + 8 + kPotentialParts * n_points * 8;
 }
@@ -591,15 +563,14 @@ cudaError_t launch_cv_potential(const SceneView<3> &s, const float4 *src, const 
                                 const float *sigma, const float *pts, uint32_t n_points, uint32_t *scratch,
                                 float *out, cudaStream_t stream) {
     if (n_points == 0) return cudaSuccess;
-    uint32_t n2 = 1;
-    while (n2 < n_points) n2 <<= 1;
+    const uint32_t n2 = sort_padded(n_points);
     uint64_t *key = (uint64_t *)scratch;
     uint32_t *bb = scratch + 2 * (size_t)n2;
     bounds_init_kernel<<<1, 32, 0, stream>>>(bb);
     pts_bounds_kernel<<<(n_points + 255) / 256, 256, 0, stream>>>(pts, n_points, bb);
     pts_morton_kernel<<<(n2 + 255) / 256, 256, 0, stream>>>(pts, n_points, n2, bb, key);
-    for (uint32_t k = 2; k <= n2; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) bitonic_kernel<<<(n2 + 255) / 256, 256, 0, stream>>>(n2, j, k, key);
+    const cudaError_t e = launch_sort_keys(n2, key, nullptr, stream);
+    if (e != cudaSuccess) return e;
     double *part_sums = reinterpret_cast<double *>(scratch + 2 * (size_t)n2 + 8);
     cv_sum_kernel<1><<<dim3((n_points + 31) / 32, kPotentialParts), kCvBlock, 0, stream>>>(
         s, src, near2, sigma, clusters, pts, key, n_points, 0.0f, out, part_sums);

@@ -4,7 +4,7 @@
 //
 // One thread running it is a chain of four dependent additions and a load per element: 33.6 ms for
 // the two tables of 327,680 triangles, nearly all of a device scene build. Here it runs in parallel
-// by speculation and is then verified, 0.11 ms for the same tables.
+// by speculation and is then verified, 0.20 ms for the same tables.
 //
 // While |s| >= |y| the step is exact apart from the rounding of y, so the pair (s, c) is the single
 // number v = s - c (s is v rounded to float) and the recurrence is
@@ -32,8 +32,8 @@
 // Then the division by the total and the nondecreasing fix-up (a prefix maximum: the division is
 // monotone, so the maximum is taken on the sums).
 //
-// Cost: kRounds + 1 passes over a chunk (about 9 ns an element, the latency of the chain) and kRounds
-// compositions (about 30 ns a chunk), so the chunk length grows with sqrt(n). Up to kSerialMax
+// Cost: kRounds + 1 passes over a chunk (about 20 ns an element, the latency of the chain) and kRounds
+// compositions (about 95 ns a chunk), so the chunk length grows with sqrt(n). Up to kSerialMax
 // elements the serial chain on one warp costs less than the launches of the other route.
 // This unit is compiled without contraction: every step is a plain IEEE addition.
 #include "kahan_scan.hpp"
@@ -358,7 +358,8 @@ __global__ void __launch_bounds__(32) kahan_serial(KahanArgs g) {
     }
 }
 
-// Chunk length: a power of two near sqrt(2.5 n), the least of (kRounds + 1) 9 ns C + kRounds 30 ns n / C.
+// Chunk length: a power of two from sqrt(1.25 n) up, about the least of (kRounds + 1) 20 ns C +
+// kRounds 95 ns n / C.
 uint32_t chunk_length(uint32_t n) {
     uint32_t C = 2 * kWindow;
     while (C < 32768u && (double)C * C < 1.25 * (double)n) C <<= 1;

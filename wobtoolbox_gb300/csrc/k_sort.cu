@@ -4,8 +4,8 @@
 // One launch per compare-exchange step (190 for 2^19 keys, 136 for 2^16) is bound by the launches: a
 // step over keys that sit in the L2 takes as long as starting it, 2.9 us. Here a block sorts and
 // merges tiles of kTile keys in shared memory, all steps of distance below kTile in one launch, and
-// the longer steps go two to a launch with four keys a thread: 24 launches for 2^19 keys (0.79 ->
-// 0.13 ms) and 11 for 2^16 (0.40 -> 0.04 ms).
+// the longer steps go two to a launch with four keys a thread: 24 launches for 2^19 keys with values
+// (0.79 -> 0.21 ms) and 11 for 2^16 without (0.40 -> 0.09 ms).
 #include "sort_keys.hpp"
 
 namespace wobgb {

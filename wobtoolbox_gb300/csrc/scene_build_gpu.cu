@@ -460,6 +460,31 @@ __global__ void k_records(uint32_t n, const uint32_t *__restrict__ val, const fl
     }
 }
 
+// New boundary data of existing records: are all offsets finite (and below 3e38)?
+__global__ void k_check_offsets(uint32_t n, const float *__restrict__ delta, uint32_t *bad) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && !(fabsf(delta[i]) <= 3.0e38f)) *bad = 1u;
+}
+// Adds offset i to record i's vertex boundary values and recomputes its |g| weight with the host
+// build's operations; nothing where a check failed.
+template <int D>
+__global__ void k_offset_weights(uint32_t n, const float *__restrict__ delta, const uint32_t *__restrict__ bad,
+                                 float *__restrict__ elems, const float4 *__restrict__ aux, float *__restrict__ bvw) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || *bad) return;
+    const float d = delta[i];
+    float *r = elems + (size_t)i * 16 + (D == 2 ? 6 : 12);
+    float s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+        const float g = r[k] + d;
+        r[k] = g;
+        s = k == 0 ? fabsf(g) : s + fabsf(g);
+    }
+    const float area = D == 2 ? elems[(size_t)i * 16 + 10] : aux[i].w;
+    bvw[i] = area * s / (float)D;
+}
+
 // The build's scratch, one allocation: take() first adds up the sizes, after allocate() it hands out
 // the pointers in the same order.
 struct Tmp {
@@ -636,6 +661,26 @@ std::string build_impl(uint32_t n, const float *verts, const float *normals, con
 }
 
 }  // namespace
+
+size_t offset_scratch_bytes(uint32_t n) { return 256 + ((size_t)n * 4 + 255) / 256 * 256 + kahan_scratch_bytes(n, 1); }
+
+cudaError_t launch_boundary_offsets(int dim, uint32_t n, const float *delta, float *elems, const float4 *aux,
+                                    float *bv_cdf, uint32_t G, uint32_t *bv_guide, void *scratch, cudaStream_t st) {
+    uint32_t *head = (uint32_t *)scratch;  // OffsetResult
+    float *bvw = (float *)((char *)scratch + 256);
+    void *kahan = (char *)scratch + 256 + ((size_t)n * 4 + 255) / 256 * 256;
+    cudaError_t e = cudaMemsetAsync(head, 0, sizeof(OffsetResult), st);
+    if (e != cudaSuccess) return e;
+    k_check_offsets<<<blocks(n), kT, 0, st>>>(n, delta, head);
+    if (dim == 2) k_offset_weights<2><<<blocks(n), kT, 0, st>>>(n, delta, head, elems, aux, bvw);
+    else k_offset_weights<3><<<blocks(n), kT, 0, st>>>(n, delta, head, elems, aux, bvw);
+    const float *w[1] = {bvw};
+    float *cdf[1] = {bv_cdf};
+    if ((e = cudaGetLastError()) != cudaSuccess ||
+        (e = launch_kahan_cdf(n, 1, w, cdf, (float *)(head + 1), kahan, st)) != cudaSuccess)
+        return e;
+    return launch_guide(n, G, bv_cdf, bv_guide, st);
+}
 
 void DeviceSceneBuild::release() {
     for (void **p : {&elems, &elem_aux, &isect, &nodes, &area_cdf, &area_guide, &bv_cdf, &bv_guide}) {

@@ -29,4 +29,16 @@ std::string build_device_scene(int dim, uint32_t n, const float *verts, const fl
                                const float *alphas, const int32_t *types, cudaStream_t stream, DeviceSceneBuild &out,
                                cudaError_t &cuda_error);
 
+// Adds delta[i] (device) to the vertex boundary values of element record i and rebuilds the |g|
+// weights' CDF (n entries) and guide table (G = min(n, 2^22) records) in new buffers, with the bits
+// of the host build. The first bytes of scratch (offset_scratch_bytes, 256-byte aligned) receive an
+// OffsetResult; where an offset is not finite the records stay as they were.
+struct OffsetResult {
+    uint32_t bad;
+    float total;
+};
+size_t offset_scratch_bytes(uint32_t n);
+cudaError_t launch_boundary_offsets(int dim, uint32_t n, const float *delta, float *elems, const float4 *aux,
+                                    float *bv_cdf, uint32_t G, uint32_t *bv_guide, void *scratch, cudaStream_t st);
+
 }  // namespace wobgb

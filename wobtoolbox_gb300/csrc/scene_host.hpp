@@ -84,16 +84,22 @@ struct HostScene {
     bool bv_valid = false;                 // |g| sampling defined (total |g| finite and > 0)
     uint32_t n_nodes = 0, depth = 0;
     LineGrid line_grid;                    // 2D only
+    bool host_built = false;
+
+    // Frees what only the upload reads: the records, the tree, the tables and the grid's lists (the
+    // storage order and the scalars stay).
+    void release_tables() {
+        for (std::vector<float> *v : {&elems, &elem_aux, &isect, &nodes, &area_cdf, &bv_cdf, &line_grid.bins})
+            std::vector<float>().swap(*v);
+        for (std::vector<uint32_t> *v : {&area_guide, &bv_guide, &line_grid.offsets}) std::vector<uint32_t>().swap(*v);
+        std::vector<uint16_t>().swap(line_grid.entries);
+    }
 };
 
 // Returns "" on success, else a message. Arrays as documented for wob_scene_create.
 std::string build_host_scene(int dim, uint32_t n, const float *verts, const float *normals,
                              const float *bvals, const float *alphas, const int32_t *types,
                              HostScene &out);
-
-// Recomputes the |g| sampling weights, CDF, guide table, total and validity from the boundary
-// values in the stored element records (after the values changed).
-void rebuild_bv_tables(HostScene &s);
 
 // Guide table of a nondecreasing CDF with G = min(n, 2^22) entries of 4 words each:
 // {lo, hi, bits(cdf[lo]), bits(cdf[lo + 1])}, where lo is the first index whose CDF value reaches
