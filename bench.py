@@ -424,7 +424,7 @@ def run_ours(args):
             # scene's sizes (L2-resident), measured now on this GPU (wob_measure_gather_peak)
             import ctypes as C
             sps, gms = C.c_double(0.0), C.c_float(0.0)
-            wob.check(wob.load().wob_measure_gather_peak(scene.n_elems, min(scene.n_elems, 1 << 22), 4096,
+            wob.check(wob.load().wob_measure_gather_peak(scene.n_elems, max(scene.n_elems, min(4 * scene.n_elems, 1 << 20)), 4096,
                                                          C.byref(sps), C.byref(gms)))
             per_sample = bytes_per_bounce / 2  # two uniform samples per bounce
             gather = {"samples_per_s": sps.value, "ms": gms.value,

@@ -98,7 +98,7 @@ struct wob_scene_s {
     wobgb::HostScene host;
     DevBuf elems, elem_aux, isect, nodes, area_cdf, area_guide, bv_cdf, bv_guide, err;
     DevBuf vol_values, vol_cdf, vol_guide;
-    DevBuf lg_bins, lg_off, lg_ent;  // 2D line grid
+    DevBuf lg_bins, lg_off, lg_ent, lg_seg;  // 2D line grid
     DevBuf cv_table;  // control-variate density per stored element
     DevBuf rhs;       // multi-RHS data [n][dim][n_rhs], storage order
     DevBuf rhs_cv;    // multi-RHS control variate [n][n_rhs], storage order
@@ -135,6 +135,7 @@ struct wob_scene_s {
         v.lg_bins = (const float4 *)lg_bins.ptr;
         v.lg_off = (const uint32_t *)lg_off.ptr;
         v.lg_ent = (const uint16_t *)lg_ent.ptr;
+        v.lg_seg = (const float4 *)lg_seg.ptr;
         v.lg_K = lg_bins.ptr ? host.line_grid.K : 0u;
         v.lg_M = host.line_grid.M;
         v.lg_cx = host.line_grid.cx;
@@ -157,7 +158,7 @@ struct wob_scene_s {
     ~wob_scene_s() { release_all(); }
     void release_all() {
         for (DevBuf *b : {&elems, &elem_aux, &isect, &nodes, &area_cdf, &area_guide, &bv_cdf, &bv_guide, &err, &vol_values,
-                          &vol_cdf, &vol_guide, &cv_table, &rhs, &rhs_cv, &ws, &lg_bins, &lg_off, &lg_ent})
+                          &vol_cdf, &vol_guide, &cv_table, &rhs, &rhs_cv, &ws, &lg_bins, &lg_off, &lg_ent, &lg_seg})
             b->release();
         if (ws_stream) cudaStreamDestroy(ws_stream);
         ws_stream = nullptr;
@@ -173,8 +174,8 @@ struct wob_batch_s {
     uint32_t n_scenes = 0;
     uint64_t total_units = 0;
     uint32_t total_points = 0;
-    uint32_t cls_first[3] = {0, 0, 0}, cls_count[3] = {0, 0, 0};
-    uint64_t cls_units[3] = {0, 0, 0};
+    uint32_t cls_first[wobgb::kBatchClasses] = {}, cls_count[wobgb::kBatchClasses] = {};
+    uint64_t cls_units[wobgb::kBatchClasses] = {};
     DevBuf table;
     ~wob_batch_s() { table.release(); }
 };
@@ -312,6 +313,16 @@ int wob_device_info(int *device, int *sm_count) {
     return WOB_OK;
 }
 
+// The 2D segments' endpoints packed from the element records.
+static cudaError_t pack_segments(wob_scene_s *s) {
+    if (s->host.line_grid.K == 0) return cudaSuccess;
+    const size_t bytes = (size_t)s->host.n * 16;
+    cudaError_t e = cudaMalloc(&s->lg_seg.ptr, bytes);
+    if (e != cudaSuccess) return e;
+    s->lg_seg.bytes = bytes;
+    return cudaMemcpy2D(s->lg_seg.ptr, 16, s->elems.ptr, 64, 16, s->host.n, cudaMemcpyDeviceToDevice);
+}
+
 static int scene_create_impl(int dim, uint32_t n_elems, const float *vertices, const float *normals,
                              const float *boundary_values, const float *robin_alphas, const int32_t *boundary_types,
                              wob_scene *out) {
@@ -345,7 +356,8 @@ static int scene_create_impl(int dim, uint32_t n_elems, const float *vertices, c
         (e = upload(s->err, &zero, 4)) != cudaSuccess ||
         (e = upload(s->lg_bins, h.line_grid.bins.data(), h.line_grid.bins.size() * 4)) != cudaSuccess ||
         (e = upload(s->lg_off, h.line_grid.offsets.data(), h.line_grid.offsets.size() * 4)) != cudaSuccess ||
-        (e = upload(s->lg_ent, h.line_grid.entries.data(), h.line_grid.entries.size() * 2)) != cudaSuccess) {
+        (e = upload(s->lg_ent, h.line_grid.entries.data(), h.line_grid.entries.size() * 2)) != cudaSuccess ||
+        (e = pack_segments(s)) != cudaSuccess) {
         s->release_all();
         return fail_cuda(e, "uploading the scene");
     }
@@ -443,7 +455,7 @@ int wob_scene_get_info(wob_scene s, wob_scene_info *info) {
     info->has_volume_cache = s->has_volume ? 1 : 0;
     size_t bytes = 0;
     for (const DevBuf *b : {&s->elems, &s->elem_aux, &s->isect, &s->nodes, &s->area_cdf, &s->area_guide, &s->bv_cdf, &s->bv_guide,
-                            &s->vol_values, &s->vol_cdf, &s->vol_guide, &s->lg_bins, &s->lg_off, &s->lg_ent})
+                            &s->vol_values, &s->vol_cdf, &s->vol_guide, &s->lg_bins, &s->lg_off, &s->lg_ent, &s->lg_seg})
         bytes += b->bytes;
     info->bytes_on_device = (uint32_t)(bytes > 0xFFFFFFFFu ? 0xFFFFFFFFu : bytes);
     info->line_grid_bins = s->lg_bins.ptr ? s->host.line_grid.K : 0u;
@@ -858,7 +870,7 @@ static int batch_create_impl(const wob_scene *scenes, const wob_params *params, 
     auto group = [b](auto &t) {
         std::stable_sort(t.begin(), t.end(), [](const auto &x, const auto &y) { return x.cls < y.cls; });
         uint32_t first = 0;
-        for (uint32_t c = 0; c < 3; c++) {
+        for (uint32_t c = 0; c < wobgb::kBatchClasses; c++) {
             uint64_t u = 0;
             uint32_t k = first;
             while (k < t.size() && t[k].cls == c) {
@@ -896,7 +908,7 @@ int wob_batch_solve(wob_batch b, const float *points, double *sum, double *sumsq
     if (!points || !sum) return fail(WOB_ERR_INVALID_ARGUMENT, "points and sum are required");
     DeviceGuard g(b->device);
     cudaError_t e = cudaSuccess;
-    for (uint32_t c = 0; c < 3 && e == cudaSuccess; c++) {
+    for (uint32_t c = 0; c < wobgb::kBatchClasses && e == cudaSuccess; c++) {
         if (b->cls_count[c] == 0 || b->cls_units[c] == 0) continue;
         e = b->dim == 2
             ? wobgb::launch_batch_2d((const wobgb::BatchEntry<2> *)b->table.ptr + b->cls_first[c], b->cls_count[c], c,
@@ -973,7 +985,7 @@ int scene_clone_impl(wob_scene src, wob_scene *out) {
     for (auto b : {&wob_scene_s::elem_aux, &wob_scene_s::isect, &wob_scene_s::nodes, &wob_scene_s::area_cdf,
                    &wob_scene_s::area_guide, &wob_scene_s::bv_cdf, &wob_scene_s::bv_guide, &wob_scene_s::vol_values,
                    &wob_scene_s::vol_cdf, &wob_scene_s::vol_guide, &wob_scene_s::lg_bins, &wob_scene_s::lg_off,
-                   &wob_scene_s::lg_ent})
+                   &wob_scene_s::lg_ent, &wob_scene_s::lg_seg})
         share(s->*b, src->*b);
     cudaError_t e = clone_buf(s->elems, src->elems);
     if (e != cudaSuccess) {
@@ -999,7 +1011,7 @@ int scene_add_boundary_offsets_impl(wob_scene s, const float *delta, uint32_t n,
     // scene's once the offsets are known to be finite (a clone's source keeps the shared old ones)
     DevBuf scratch, cdf, guide;
     wobgb::HostScene &h = s->host;
-    const uint32_t G = std::min<uint32_t>(n, 1u << 22);
+    const uint32_t G = wobgb::guide_records(n);
     const size_t work = wobgb::offset_scratch_bytes(n);
     auto alloc = [](DevBuf &b, size_t bytes) {
         const cudaError_t r = cudaMalloc(&b.ptr, bytes);

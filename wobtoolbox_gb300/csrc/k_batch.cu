@@ -1,6 +1,7 @@
 // Batched walk: many scenes, each with its own parameters and evaluation points, in one persistent
-// launch per walk class (at most three: backward single layer, forward single-layer Neumann, and
-// the general walk). A device table holds, per scene, its scene view, walk parameters and first
+// launch per walk class (at most five: backward single layer and forward single-layer Neumann, each
+// with and without a source term, and the general walk, whose code for every model and estimator
+// stalls on instruction fetches: 2.2 cycles an instruction where the sources ran in it). A device table holds, per scene, its scene view, walk parameters and first
 // work unit; warps take units in a grid-stride loop and find their scene by bisection over the
 // units' prefix. A unit is 32 * ppt paths of one point of one scene, so a warp never mixes scenes,
 // and the per-scene work is exactly what a single-scene launch does (same walker variant, same
@@ -9,13 +10,16 @@
 
 namespace wobgb {
 
+constexpr int kBatchMinB = 8;  // 24 scenes: 12.6 ms at 5, 11.3 at 6, 11.1 at 8
+
 // One unit (32 * ppt paths of one point) of a batched scene with the walker variant W; view and
 // p are the scene's view and parameters staged in shared memory by the warp.
 template <int D, class W>
 __device__ __forceinline__ void batch_unit(const BatchEntry<D> &e, const SceneView<D> &view, const WalkParams &p,
                                            uint32_t lane, uint64_t local, const float *__restrict__ pts,
                                            double *__restrict__ sum, double *__restrict__ sumsq,
-                                           uint64_t path_offset_add, unsigned long long &my_bounces) {
+                                           uint64_t path_offset_add, unsigned long long &my_bounces,
+                                           double (*acc)[kBlock]) {
     const uint32_t pt = (uint32_t)(local / e.slabs);
     const uint32_t span = 32u * p.ppt;
     const uint32_t first = (uint32_t)(local % e.slabs) * span;
@@ -23,9 +27,9 @@ __device__ __forceinline__ void batch_unit(const BatchEntry<D> &e, const SceneVi
     V<D> x;
 #pragma unroll
     for (int i = 0; i < D; i++) x.v[i] = __ldg(pts + (size_t)row * D + i);
-    double acc[D + 1], acc2[D + 1];
+    const uint32_t tid = threadIdx.x;  // this thread's running sums (c) and sums of squares (D + 1 + c)
 #pragma unroll
-    for (int c = 0; c <= D; c++) { acc[c] = 0.0; acc2[c] = 0.0; }
+    for (int c = 0; c < 2 * (D + 1); c++) acc[c][tid] = 0.0;
     for (uint32_t k = 0; k < p.ppt; k++) {
         const uint32_t path = first + k * 32u + lane;
         if (path < p.n_paths) {
@@ -36,16 +40,16 @@ __device__ __forceinline__ void batch_unit(const BatchEntry<D> &e, const SceneVi
 #pragma unroll
             for (int c = 0; c <= D; c++) {
                 const double v = (double)out[c];
-                acc[c] += v;
-                acc2[c] += v * v;
+                acc[c][tid] += v;
+                acc[D + 1 + c][tid] += v * v;
             }
         }
     }
     __syncwarp();
 #pragma unroll
     for (int c = 0; c <= D; c++) {
-        const double sv = warp_sum(acc[c]);
-        const double qv = warp_sum(acc2[c]);
+        const double sv = warp_sum(acc[c][tid]);
+        const double qv = warp_sum(acc[D + 1 + c][tid]);
         if (lane == 0) {
             atomicAdd(sum + (size_t)row * (D + 1) + c, sv);
             if (sumsq) atomicAdd(sumsq + (size_t)row * (D + 1) + c, qv);
@@ -57,7 +61,7 @@ __device__ __forceinline__ void batch_unit(const BatchEntry<D> &e, const SceneVi
 // (the specialisation a single-scene launch of that class uses); a warp finds its scene by
 // bisection over the units' prefix.
 template <int D, class W>
-__global__ void __launch_bounds__(kBlock) batch_domain_kernel(const BatchEntry<D> *__restrict__ table,
+__global__ void __launch_bounds__(kBlock, kBatchMinB) batch_domain_kernel(const BatchEntry<D> *__restrict__ table,
                                                               uint32_t n_scenes, uint64_t total_units,
                                                               const float *__restrict__ pts, double *__restrict__ sum,
                                                               double *__restrict__ sumsq,
@@ -65,6 +69,7 @@ __global__ void __launch_bounds__(kBlock) batch_domain_kernel(const BatchEntry<D
                                                               uint64_t path_offset_add) {
     __shared__ SceneView<D> s_view[kBlock / 32];
     __shared__ WalkParams s_params[kBlock / 32];
+    __shared__ double s_acc[2 * (D + 1)][kBlock];
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t n_warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -90,7 +95,7 @@ __global__ void __launch_bounds__(kBlock) batch_domain_kernel(const BatchEntry<D
             staged = lo;
         }
         batch_unit<D, W>(e, s_view[wib], s_params[wib], lane, u - e.unit_begin, pts, sum, sumsq, path_offset_add,
-                         my_bounces);
+                         my_bounces, s_acc);
     }
     if (bounces) {
         __syncwarp();
@@ -121,6 +126,13 @@ cudaError_t launch_batch_impl(const BatchEntry<D> *table, uint32_t n_scenes, uin
         return launch_class<D, Walker<D, kSingleLayer, kStratFwdSlNeumann, false, true>>(table, n_scenes, total_units, pts,
                                                                                     sum, sumsq, bounces, path_offset_add,
                                                                                     stream);
+    if (cls == 3u)
+        return launch_class<D, Walker<D, kSingleLayer, kStratSingleLayer, true, true>>(table, n_scenes, total_units, pts, sum,
+                                                                                  sumsq, bounces, path_offset_add, stream);
+    if (cls == 4u)
+        return launch_class<D, Walker<D, kSingleLayer, kStratFwdSlNeumann, true, true>>(table, n_scenes, total_units, pts,
+                                                                                   sum, sumsq, bounces, path_offset_add,
+                                                                                   stream);
     return launch_class<D, Walker<D, -1, kStratRuntime, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
                                                                 path_offset_add, stream);
 }

@@ -20,7 +20,7 @@ constexpr uint32_t kStreamVpl = 2u;
 constexpr int kVplTile = 256;
 
 template <int D>
-__global__ void __launch_bounds__(kBlock) vpl_paths_kernel(SceneView<D> s, WalkParams p, uint32_t n_paths,
+__global__ void __launch_bounds__(kBlock, 6) vpl_paths_kernel(SceneView<D> s, WalkParams p, uint32_t n_paths,
                                                            float *__restrict__ vpl_p, float *__restrict__ vpl_mu,
                                                            unsigned long long *__restrict__ bounces) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

@@ -17,7 +17,7 @@ size_t kahan_scratch_bytes(uint32_t n, int arrays);
 cudaError_t launch_kahan_cdf(uint32_t n, int arrays, const float *const *w, float *const *cdf, float *totals,
                              void *scratch, cudaStream_t stream);
 
-// Guide table (scene_build.cpp's build_guide) of a nondecreasing device CDF: G = min(n, 2^22)
+// Guide table (scene_build.cpp's build_guide) of a nondecreasing device CDF: G = guide_records(n)
 // records of 4 words.
 cudaError_t launch_guide(uint32_t n, uint32_t G, const float *cdf, uint32_t *rec, cudaStream_t stream);
 

@@ -146,8 +146,7 @@ bool finite_all(const float *p, size_t n) {
 
 std::vector<uint32_t> build_guide(const std::vector<float> &cdf) {
     const uint32_t n = (uint32_t)cdf.size();
-    uint32_t G = std::min<uint32_t>(n, 1u << 22);
-    if (G == 0) G = 1;
+    const uint32_t G = guide_records(n);
     std::vector<uint32_t> first(G);
     uint32_t i = 0;
     for (uint32_t j = 0; j < G; j++) {

@@ -640,7 +640,7 @@ std::string build_impl(uint32_t n, const float *verts, const float *normals, con
     out.total_area = hb.totals[0];
     out.total_bv = hb.totals[1];
     if (!(out.total_area > 0.0f) || !std::isfinite(out.total_area)) return "total boundary area must be positive and finite";
-    const uint32_t G = std::max<uint32_t>(1u, std::min<uint32_t>(n, 1u << 22));
+    const uint32_t G = guide_records(n);
     uint32_t *ag = nullptr, *bg = nullptr;
     WOB_CK(cudaMalloc(&ag, (size_t)G * 16));
     out.area_guide = ag;

@@ -30,7 +30,7 @@ std::string build_device_scene(int dim, uint32_t n, const float *verts, const fl
                                cudaError_t &cuda_error);
 
 // Adds delta[i] (device) to the vertex boundary values of element record i and rebuilds the |g|
-// weights' CDF (n entries) and guide table (G = min(n, 2^22) records) in new buffers, with the bits
+// weights' CDF (n entries) and guide table (G = guide_records(n) records) in new buffers, with the bits
 // of the host build. The first bytes of scratch (offset_scratch_bytes, 256-byte aligned) receive an
 // OffsetResult; where an offset is not finite the records stay as they were.
 struct OffsetResult {

@@ -101,7 +101,19 @@ std::string build_host_scene(int dim, uint32_t n, const float *verts, const floa
                              const float *bvals, const float *alphas, const int32_t *types,
                              HostScene &out);
 
-// Guide table of a nondecreasing CDF with G = min(n, 2^22) entries of 4 words each:
+// Records of the guide table of n CDF entries: 4 per entry up to 2^20 records, then one per entry, at
+// most 2^22 (key G then keeps its rounding under a quarter bin). With one record per entry a lookup
+// spans two bins and on average two boundaries, and in most warps some lane falls through the
+// record's two CDF values into the bisection's dependent loads; with four per entry that is rare: the
+// Robin walk on 81,920 triangles went from 25.7 to 24.4 ms (37.5 to 29.4 without a register cap), 64-candidate resampling for 64 right-hand sides from
+// 2.43 to 2.06 ms. Above 2^20 records the table would crowd the element records out of the L2.
+inline uint32_t guide_records(uint32_t n) {
+    const uint64_t four = 4 * (uint64_t)n, wide = four < (1u << 20) ? four : (1u << 20);
+    const uint64_t g = wide > n ? wide : n;
+    return g < 1 ? 1u : g < (1u << 22) ? (uint32_t)g : (1u << 22);
+}
+
+// Guide table of a nondecreasing CDF with G = guide_records(n) entries of 4 words each:
 // {lo, hi, bits(cdf[lo]), bits(cdf[lo + 1])}, where lo is the first index whose CDF value reaches
 // (j - 1/2)/G and hi the lo of entry j + 2 (n - 1 for the last two). See cdf_search in
 // device_common.cuh for why the answer for a key in bin j lies in [lo, hi].

@@ -40,7 +40,15 @@ template <> struct Green<2> {
         return vdiv(vscale(0x1.45f306p-3f, vnormalized(r)), fmax_ref(vnorm(r), eps));
     }
     __device__ __forceinline__ float dG_dny(const V<2> &y, const V<2> &x, const V<2> &ny) const {
+        // (r / |r|) . n / max(|r|, eps): three quotients by |r| unless eps is larger
         const V<2> r = vsub(y, x);
+        const float z = vsqnorm(r), s = sqrtf(z);
+        if (__builtin_expect(s >= eps && mid_magnitude(s) && zero_or_not_tiny(r.v[0]) && zero_or_not_tiny(r.v[1]), 1)) {
+            const SharedDivisor d = shared_divisor(s);
+            const V<2> rh{{shared_quotient(r.v[0], d), shared_quotient(r.v[1], d)}};
+            const float num = -0x1.45f306p-3f * vdot(rh, ny);
+            if (zero_or_not_tiny(num)) return shared_quotient(num, d);
+        }
         return -0x1.45f306p-3f * vdot(vnormalized(r), ny) / fmax_ref(vnorm(r), eps);
     }
     __device__ __forceinline__ V<2> d2G_dxdny(const V<2> &y, const V<2> &x, const V<2> &ny) const {
@@ -314,13 +322,40 @@ template <int D, int kBie = -1, int kStrat = kStratRuntime, bool kVol = true, bo
     __device__ __forceinline__ bool direct_neumann() const { return strat() == kStratDirectNeumann; }
     __device__ __forceinline__ bool sl_neumann() const { return strat() == kStratFwdSlNeumann; }
 
+    // |G| at a Dirichlet point, |dG/dn| at a Neumann point, |dG/dn + alpha G| at a Robin point, with the
+    // operations of Green's functions; in 3D the first two share their final division, so the lanes
+    // of a warp whose points differ in type do not run one after the other.
     __device__ __forceinline__ float ris_target_at(int type, const BPoint<D> &yp, const V<D> &c) const {
-        if (type == kDirichlet) return fabsf(K.G(c, yp.p));
-        if (type == kNeumann) return fabsf(K.dG_dny(yp.p, c, yp.n));
-        return fabsf(K.dG_dny(yp.p, c, yp.n) + yp.alpha * K.G(c, yp.p));
+        if constexpr (D == 3) {
+            const V<3> r = vsub(yp.p, c);
+            const float z = vsqnorm(r), n = sqrtf(z);
+            const float gden = 0x1.921fb6p+3f * fmax_ref(n, p.eps);
+            float num = 1.0f, den = gden;
+            if (type != kDirichlet) {
+                const V<3> rh = z > 0.0f ? vdiv_norm(r, n) : r;
+                num = -0x1.45f306p-4f * vdot(rh, yp.n);
+                den = fmax_ref(z, p.eps);
+            }
+            float v = num / den;
+            if (type == kRobin) v = v + yp.alpha * (1.0f / gden);
+            return fabsf(v);
+        } else {
+            if (type == kDirichlet) return fabsf(K.G(c, yp.p));
+            if (type == kNeumann) return fabsf(K.dG_dny(yp.p, c, yp.n));
+            return fabsf(K.dG_dny(yp.p, c, yp.n) + yp.alpha * K.G(c, yp.p));
+        }
     }
     __device__ __forceinline__ float ris_target(int type, const BPoint<D> &yp, const BPoint<D> &c) const {
         return ris_target_at(type, yp, c.p);
+    }
+    // r <= w / sum (the rounded quotient), without the division unless r sum lies within 2^-22 of w.
+    // A first product p = r sum (1 + 2^-24) below w (1 - 2^-22) puts r below the quotient by more than
+    // its rounding, one above w (1 + 2^-22) above it; p is normal for r >= 2^-24 and sum > 1e-30.
+    static __device__ __forceinline__ bool at_most_ratio(float r, float w, float sum) {
+        const float prod = r * sum;
+        const bool below = prod < w * 0x1.fffff8p-1f, above = prod > w * 0x1.000004p+0f;
+        if (__builtin_expect(sum > 1e-30f && (below || above), 1)) return below;
+        return r <= w / sum;
     }
     // Streaming RIS over K uniform candidates (scene.cuh:542-584, 847-889). A candidate's target
     // needs only its position, so the loop reads only the vertices of each candidate's element and
@@ -328,6 +363,12 @@ template <int D, int kBie = -1, int kStrat = kStratRuntime, bool kVol = true, bo
     // are taken in the reference's order -- candidate i's D draws, then its selection draw -- but
     // candidate i + 1's draws and guide-table load are issued before candidate i's target is
     // evaluated, so two dependent load chains are in flight instead of one.
+    //
+    // The loop is bound by issue and by the latency of its serial operations (3 "wait" stall cycles
+    // per instruction at 20 warps per SM). A candidate's D + 1 draws come from a window of two Philox
+    // blocks at one position, so a candidate costs one block at one call site instead of a refill
+    // check and a copy of the generator at each draw; the selection needs no division; and the
+    // target's quotients share reciprocals.
     __device__ __forceinline__ void ris_select(const BPoint<D> &yp, uint32_t &sel, float *su, float &w_sum,
                                                uint32_t &M) {
         sel = 0xFFFFFFFFu;
@@ -337,33 +378,65 @@ template <int D, int kBie = -1, int kStrat = kStratRuntime, bool kVol = true, bo
         M = 0;
         const uint32_t K = p.n_resampling;
         if (K == 0) return;
-        float u[D];
-#pragma unroll
-        for (int k = 0; k < D; k++) u[k] = rng.uniform();
+        auto block = [&](uint32_t b) { return philox4x32_10(make_uint4(b, rng.c1, rng.c2, rng.c3), rng.k0, rng.k1); };
+        uint4 cur = rng.buf;         // the block holding the next draw, at position pos
+        uint32_t pos = (uint32_t)rng.used, next_block = rng.block;
+        if (pos == 4u) {
+            cur = block(next_block++);
+            pos = 0;
+        }
+        uint4 nxt = block(next_block++);
+        auto take = [&](float *u, float &r_sel) {
+            const bool odd = pos & 1u, high = pos & 2u;
+            auto pick = [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+                const uint32_t x = high ? (odd ? d : c) : (odd ? b : a);
+                return (float)((x >> 8) + 1u) * 0x1p-24f;
+            };
+            u[0] = pick(cur.x, cur.y, cur.z, cur.w);
+            u[1] = pick(cur.y, cur.z, cur.w, nxt.x);
+            if constexpr (D == 2) {
+                r_sel = pick(cur.z, cur.w, nxt.x, nxt.y);
+                pos += 3u;
+            } else {
+                u[2] = pick(cur.z, cur.w, nxt.x, nxt.y);
+                r_sel = pick(cur.w, nxt.x, nxt.y, nxt.z);
+                pos += 4u;
+            }
+            if (pos >= 4u) {
+                pos -= 4u;
+                cur = nxt;
+                nxt = block(next_block++);
+            }
+        };
+        float u[D], r_sel;
+        take(u, r_sel);
         uint4 g = __ldg(s.area_guide + guide_bin(s.area_G, u[0]));
         for (uint32_t i = 0; i < K; i++) {
             const uint32_t idx = cdf_resolve(s.area_cdf, g, u[0]);
-            const V<D> pos = uniform_position<D>(s, idx, u);
-            const float r_sel = rng.uniform();
-            float un[D];
+            const V<D> at = uniform_position<D>(s, idx, u);
+            float un[D], rn = 0.0f;
 #pragma unroll
             for (int k = 0; k < D; k++) un[k] = 0.0f;
             if (i + 1 < K) {
-#pragma unroll
-                for (int k = 0; k < D; k++) un[k] = rng.uniform();
+                take(un, rn);
                 g = __ldg(s.area_guide + guide_bin(s.area_G, un[0]));
             }
-            const float wi = ris_target_at(yp.type, yp, pos) * s.total_area;
+            const float wi = ris_target_at(yp.type, yp, at) * s.total_area;
             w_sum = w_sum + wi;
-            M += 1;
-            if (r_sel <= wi / w_sum) {
+            if (at_most_ratio(r_sel, wi, w_sum)) {
                 sel = idx;
 #pragma unroll
                 for (int k = 0; k < D; k++) su[k] = u[k];
             }
 #pragma unroll
             for (int k = 0; k < D; k++) u[k] = un[k];
+            r_sel = rn;
         }
+        M = K;
+        // the stream as K (D + 1) single draws leave it: cur is loaded, pos of its words are used
+        rng.buf = cur;
+        rng.used = (int)pos;
+        rng.block = next_block - 1u;
     }
     __device__ __forceinline__ BPoint<D> sample_ris(const BPoint<D> &yp, float &inv_pdf) {
         uint32_t sel, M;
@@ -601,12 +674,13 @@ template <int D> struct BatchEntry {
 };
 
 // The specialised walk a batched scene runs: 1 = backward single layer, 2 = forward single-layer
-// Neumann (both without a source term), 0 = the general walk.
+// Neumann, 3 and 4 the same with a source term, 0 = the general walk.
+constexpr uint32_t kBatchClasses = 5u;
 __host__ __device__ __forceinline__ uint32_t batch_walk_class(const WalkParams &p) {
-    if (p.n_volume != 0) return 0u;
+    const uint32_t vol = p.n_volume != 0 ? 2u : 0u;
     const int st = strategy_of(p.bie, p.estimator, p.problem);
-    if (st == kStratSingleLayer) return 1u;
-    if (st == kStratFwdSlNeumann) return 2u;
+    if (st == kStratSingleLayer) return 1u + vol;
+    if (st == kStratFwdSlNeumann) return 2u + vol;
     return 0u;
 }
 
