@@ -3,7 +3,8 @@
 //
 // A query tests the segments its grid cell lists: 5 on average on a 1024-segment star (41 on 8192
 // segments) but up to 40, so a lane per query ran at 13 of 32 lanes and 1,600 instructions a bounce
-// (6.6 ms for 7,960 points x 1024 paths x 8 bounces; 4.3 and 3.8 ms at 8 and 12 blocks per SM). Here a
+// (3.3 ms for 7,960 points x 1024 paths x 8 bounces at 12 blocks per SM; 2.46 ms for 4,000 x 256 on 8192
+// segments). This kernel takes 2.9 ms and 1.23 ms. A
 // warp lays the lists of its 32 queries end to end (a scan of their lengths) and tests 32 candidates at
 // a time, a lane each: the lane finds the query that owns its candidate from the bit mask of the
 // queries that begin in the round, fetches that query's line by shuffles, and the round's ballot is
@@ -121,6 +122,8 @@ __global__ void __launch_bounds__(kBlock, kMinB) dl2d_kernel(SceneView<2> s, Wal
                                                              float *__restrict__ per_path) {
     __shared__ uint32_t s_ballots[kBlock / 32][kBallots];
     __shared__ uint32_t s_owners[kBlock / 32][32];
+    __shared__ double acc[6][kBlock];  // [c]: a thread's running sum, [3 + c]: its sum of squares
+    const uint32_t tid = threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t *ballots = s_ballots[threadIdx.x >> 5], *owners = s_owners[threadIdx.x >> 5];
     owners[lane] = 0u;
@@ -137,61 +140,58 @@ __global__ void __launch_bounds__(kBlock, kMinB) dl2d_kernel(SceneView<2> s, Wal
         V<2> x;
 #pragma unroll
         for (int i = 0; i < 2; i++) x.v[i] = __ldg(pts + (size_t)pt * 2 + i);
-        double acc[6];
 #pragma unroll
-        for (int c = 0; c < 6; c++) acc[c] = 0.0;
+        for (int c = 0; c < 6; c++) acc[c][tid] = 0.0;
         for (uint32_t k = 0; k < p.ppt; k++) {
             const uint32_t path = first + k * 32u + lane;
             const bool active = path < p.n_paths;
             DlWalker w(s, p, kStreamDomain, p.point_offset + pt, p.path_offset + path);
-            float ip;
-            const BPoint<2> y0 = warp_line_sample(w, active, x, ip, ballots, owners);
-            // compute_sample_unknown_boundary
-            float contrib = 0.0f, wt = 1.0f;
-            BPoint<2> y_prev = y0;
+            // domain(): the first sample from x and what the path's estimate multiplies there, then
+            // unknown_boundary()'s bounces, each from the sample before it
+            float contrib = 0.0f, wt = 1.0f, known = 0.0f, du = 0.0f;
+            V<2> gk = vzero<2>(), gu = vzero<2>();
+            BPoint<2> y_prev = bp_zero<2>();
+            y_prev.p = x;
             bool alive = active;
             for (uint32_t m = 0; m < L; m++) {
-                const bool last = m == L - 1;
-                BPoint<2> y = y_prev;
-                if (alive) {
-                    w.bounces++;
-                    if (last) wt = 0.5f * wt;
-                    contrib = contrib + wt * w.fbk(y_prev, y, 0.0f);
-                }
-                if (last) break;
                 if (!__any_sync(kFullWarp, alive)) break;
-                float ipm;
-                y = warp_line_sample(w, alive, y_prev.p, ipm, ballots, owners);
+                float ip;
+                BPoint<2> y = warp_line_sample(w, alive, y_prev.p, ip, ballots, owners);
                 if (alive) {
-                    wt = wt * w.fbu(y_prev, y, ipm, true);
+                    if (m == 0) {
+                        known = w.sdk(x, y, ip);
+                        du = w.sdu(x, y, ip);
+                        gk = w.gdk(x, y, ip);
+                        gu = w.gdu(x, y, ip);
+                    } else {
+                        wt = wt * w.fbu(y_prev, y, ip, true);
+                        alive = !(wt == 0.0f);
+                    }
                     y_prev = y;
-                    alive = !(wt == 0.0f);
+                    if (alive) {
+                        w.bounces++;
+                        if (m == L - 1) wt = 0.5f * wt;
+                        contrib = contrib + wt * w.fbk(y_prev, y, 0.0f);
+                    }
                 }
             }
             if (active) {
-                // sdk and gdk of the double layer are zero; out = 0 + mu sdu, mu gdu
-                float out[3];
-                out[0] = w.sdk(x, y0, ip);
-                const V<2> g = w.gdk(x, y0, ip);
-                out[0] = out[0] + contrib * w.sdu(x, y0, ip);
-                const V<2> gu = w.gdu(x, y0, ip);
-#pragma unroll
-                for (int i = 0; i < 2; i++) out[1 + i] = g.v[i] + contrib * gu.v[i];
+                const float out[3] = {known + contrib * du, gk.v[0] + contrib * gu.v[0], gk.v[1] + contrib * gu.v[1]};
                 my_bounces += w.bounces;
 #pragma unroll
                 for (int c = 0; c < 3; c++) {
                     if (kPerPath) per_path[((size_t)pt * p.n_paths + path) * 3 + c] = out[c];
                     const double v = (double)out[c];
-                    acc[c] += v;
-                    acc[3 + c] += v * v;
+                    acc[c][tid] += v;
+                    acc[3 + c][tid] += v * v;
                 }
             }
         }
         if (!kPerPath) {
 #pragma unroll
             for (int c = 0; c < 3; c++) {
-                const double sv = warp_sum(acc[c]);
-                const double qv = warp_sum(acc[3 + c]);
+                const double sv = warp_sum(acc[c][tid]);
+                const double qv = warp_sum(acc[3 + c][tid]);
                 if (lane == 0) {
                     atomicAdd(sum + (size_t)pt * 3 + c, sv);
                     if (sumsq) atomicAdd(sumsq + (size_t)pt * 3 + c, qv);
@@ -227,6 +227,12 @@ cudaError_t launch_min(const SceneView<2> &s, const WalkParams &p_in, const floa
 cudaError_t launch_dl_grid_2d(int min_blocks, const SceneView<2> &s, const WalkParams &p, const float *pts,
                               uint32_t n_points, double *sum, double *sumsq, unsigned long long *bounces,
                               float *per_path, cudaStream_t stream) {
+    // With every warp of the launch resident at 8 blocks per SM, fewer registers only cost spills (64
+    // points x 64 paths: 34 us at 8 blocks, 38 at 12; 1000 points x 200 paths, past the line: 76 and 64).
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (min_blocks > 8 && (uint64_t)n_points * ((p.n_paths + 31u) / 32u) <= (uint64_t)sms * 8u * (kBlock / 32)) min_blocks = 8;
     switch (min_blocks) {
     case 5: return launch_min<5>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
     case 8: return launch_min<8>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);

@@ -19,7 +19,8 @@ namespace {
 // Defaults, each the fastest of its configurations over sizes: the 3D direct walks at >= 8 blocks/SM
 // (81,920-triangle Robin slice, 512 paths: 24.4 ms against 25.0 at >= 5, 36.0 at >= 10 and, before, 37.8
 // without a register cap; direct Neumann on 81,920 triangles: 3.97 ms against 4.39, 4.01 and 4.52),
-// the 2D double layer at >= 12, the 3D forward walk on the wavefront (trace at >= 6 blocks/SM on
+// the 2D double layer at >= 12 (1024-segment star: 2.87 ms against 3.88, 2.95 and 2.86 at >= 5, 8 and 10;
+// 8192 segments: 1.23 against 2.00, 1.45 and 1.33), the 3D forward walk on the wavefront (trace at >= 6 blocks/SM on
 // compressed nodes, 2^22-path chunks).
 std::atomic<int> g_config[kNumTunable] = {{1}, {3}, {1}, {3}};
 const char *kFwdNames[kTuneOccupancies] = {"lockstep walk, >=5 blocks/SM", "wavefront, trace >=8 blocks/SM",
@@ -86,8 +87,16 @@ cudaError_t launch_domain_config(int dim, int variant, int config, const void *s
     if (config < 0 || config >= kTuneConfigs) config = 0;
     if (variant == 0 && dim == 3)
         return launch_cfg<3, kDirect, kStratUniform>(config, *(const SceneView<3> *)scene_view, p, pts, n, sum, sumsq, b, pp, st);
-    if (variant == 1 && dim == 2)
-        return launch_cfg<2, kDoubleLayer, kStratLineIntersection>(config, *(const SceneView<2> *)scene_view, p, pts, n, sum, sumsq, b, pp, st);
+    if (variant == 1 && dim == 2) {
+        // scenes with a line grid (host-built, up to 16,384 segments) take the warp-shared queries; the
+        // others' BVH queries stay a lane each
+        const SceneView<2> &v = *(const SceneView<2> *)scene_view;
+        WalkParams q = p;
+        q.ppt_cap = kPptCapOf[config / kTuneOccupancies];
+        if (v.lg_K != 0u)
+            return launch_dl_grid_2d(kMinBOf[config % kTuneOccupancies], v, q, pts, n, sum, sumsq, b, pp, st);
+        return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 8>(v, q, pts, n, sum, sumsq, b, pp, st);
+    }
     if (variant == 2 && dim == 3)
         return launch_cfg<3, kDirect, kStratDirectNeumann>(config, *(const SceneView<3> *)scene_view, p, pts, n, sum, sumsq, b, pp, st);
     if (variant == 3 && dim == 3) {

@@ -110,6 +110,11 @@ inline uint32_t choose_ppt(uint64_t n_points, uint32_t n_paths) {
 cudaError_t launch_fwd_wave_3d(const SceneView<3> &s, const WalkParams &p, const float *pts, uint32_t n_points,
                                double *sum, double *sumsq, unsigned long long *bounces, float *per_path, int shape,
                                uint32_t max_slots, cudaStream_t stream);
+// The 2D double-layer Dirichlet walk on a scene with a line grid, queries shared by the warp (k2_dl.cu),
+// compiled for min_blocks (5, 8, 10 or 12) resident blocks per SM.
+cudaError_t launch_dl_grid_2d(int min_blocks, const SceneView<2> &s, const WalkParams &p, const float *pts,
+                              uint32_t n_points, double *sum, double *sumsq, unsigned long long *bounces,
+                              float *per_path, cudaStream_t stream);
 // Dispatchers (kernels_dispatch.cu): pick the specialised variant for the parameters.
 cudaError_t launch_domain_2d(const SceneView<2> &s, const WalkParams &p, const float *pts, uint32_t n_points,
                              double *sum, double *sumsq, unsigned long long *bounces, float *per_path,
