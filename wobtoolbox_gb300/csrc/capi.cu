@@ -1065,7 +1065,7 @@ int scene_add_boundary_offsets_impl(wob_scene s, const float *delta, uint32_t n,
 
 // Triangle sources and clusters of sigma~ in a scratch allocation freed on return.
 struct CvSources {
-    DevBuf src, near2, clusters;
+    DevBuf src, near2, geom, clusters;
 };
 int cv_sources(wob_scene s, const float *sigma, float near_factor, float theta, CvSources &cs, cudaStream_t st) {
     if (s->host.dim != 3) return fail(WOB_ERR_UNSUPPORTED, "the control-variate tables are implemented for 3D scenes");
@@ -1076,13 +1076,14 @@ int cv_sources(wob_scene s, const float *sigma, float near_factor, float theta, 
     const size_t n_rec = wobgb::cv_cluster_records((uint32_t)n);  // clusters and their two group levels
     cudaError_t e;
     if ((e = cudaMalloc(&cs.src.ptr, n * 16)) != cudaSuccess || (e = cudaMalloc(&cs.near2.ptr, n * 4)) != cudaSuccess ||
+        (e = cudaMalloc(&cs.geom.ptr, n * 64)) != cudaSuccess ||
         (e = cudaMalloc(&cs.clusters.ptr, n_rec * 64)) != cudaSuccess)
         return fail_cuda(e, "allocating the control-variate sources");
     cs.src.bytes = n * 16;
     cs.near2.bytes = n * 4;
     cs.clusters.bytes = n_rec * 64;
     e = wobgb::launch_cv_sources(s->view<3>(), sigma, near_factor, theta, (float4 *)cs.src.ptr, (float *)cs.near2.ptr,
-                                 (float4 *)cs.clusters.ptr, st);
+                                 (float4 *)cs.geom.ptr, (float4 *)cs.clusters.ptr, st);
     return e == cudaSuccess ? WOB_OK : fail_cuda(e, "launching the control-variate sources");
 }
 }  // namespace
@@ -1161,12 +1162,14 @@ int wob_cv_residual_data(wob_scene s, const float *sigma, int domain, float near
             // c = domain_type_coefficient / integral_free_term(1/2) (bie_models.cuh:66-78)
             const float c = domain == WOB_INTERIOR_DOMAIN ? 2.0f : -2.0f;
             cudaError_t e = wobgb::launch_cv_residual(s->view<3>(), (const float4 *)cs.src.ptr, (const float *)cs.near2.ptr,
-                                                      (const float4 *)cs.clusters.ptr, sigma, c, delta, st);
+                                                      (const float4 *)cs.geom.ptr, (const float4 *)cs.clusters.ptr, sigma, c,
+                                                      delta, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) r = fail_cuda(e, "computing the residual data");
         }
         cs.src.release();
         cs.near2.release();
+        cs.geom.release();
         cs.clusters.release();
         return r;
     });
@@ -1189,7 +1192,8 @@ int wob_cv_potential(wob_scene s, const float *sigma, float near_factor, float t
             if (e == cudaSuccess) {
                 order.bytes = words * 4;
                 e = wobgb::launch_cv_potential(s->view<3>(), (const float4 *)cs.src.ptr, (const float *)cs.near2.ptr,
-                                               (const float4 *)cs.clusters.ptr, sigma, points, n_points,
+                                               (const float4 *)cs.geom.ptr, (const float4 *)cs.clusters.ptr, sigma, points,
+                                               n_points,
                                                (uint32_t *)order.ptr, out, st);
             }
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1197,6 +1201,7 @@ int wob_cv_potential(wob_scene s, const float *sigma, float near_factor, float t
         }
         cs.src.release();
         cs.near2.release();
+        cs.geom.release();
         cs.clusters.release();
         order.release();
         return r;

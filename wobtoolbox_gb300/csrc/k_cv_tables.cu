@@ -33,10 +33,10 @@
 // near ones; a near cluster is taken triangle by triangle as above. theta = 0 takes every
 // triangle (the dense sum). The decisions are uniform across the block, so lanes never diverge.
 //
-// Work decomposition: one block per 32 targets (a lane each); its 8 warps make the same decisions
-// and take the work by index (a far group to warp index mod 8, the 8 clusters of a near group one
-// each), records read as broadcasts; FP32 partial sums over 32 items, FP64 across them and across
-// the warps (in warp order: deterministic).
+// Work decomposition: one block per 32 targets (a lane each). Its threads decide the records, a record
+// each; its 8 warps take the far records, then the near clusters, then the closed forms in turn,
+// records read as broadcasts; FP32 partial sums over 32 items, FP64 across them and across the warps
+// (in warp order: deterministic).
 // This unit is compiled with FMA contraction (it is not part of the bit-exact walk).
 #include "device_common.cuh"
 #include "launch.hpp"
@@ -48,6 +48,7 @@ namespace {
 
 constexpr int kCvBlock = 256;
 constexpr int kCvWarps = kCvBlock / 32;
+constexpr uint32_t kNearList = 256;  // near triangles a warp lists; further ones it sums at once
 constexpr double kInv4Pi = 0.07957747154594767;
 
 struct TriVerts {
@@ -64,70 +65,80 @@ __device__ __forceinline__ TriVerts load_tri(const SceneView<3> &s, uint32_t i) 
     return t;
 }
 
-// ln((R+ + s+) / (R- + s-)), in the form without cancellation for the edge's side of rho.
-__device__ __forceinline__ float edge_log(float Rp, float sp, float Rm, float sm) {
-    if (sm + sp >= 0.0f) return logf((Rp + sp) / (Rm + sm));
-    return logf((Rm - sm) / (Rp - sp));
+// What the closed form needs of a triangle alone, computed once per table (TriGeom): the unit normal and
+// its length before normalisation (twice the area; 0: degenerate, no contribution), and the three
+// edges' unit directions and lengths.
+struct TriGeom {
+    float4 n, s[3];
+};
+__device__ __forceinline__ TriGeom triangle_geometry(const TriVerts &t) {
+    const float *vs[4] = {t.a, t.b, t.c, t.a};
+    TriGeom g;
+    float e[3][3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        for (int k = 0; k < 3; k++) e[i][k] = vs[i + 1][k] - vs[i][k];
+        const float l = sqrtf(e[i][0] * e[i][0] + e[i][1] * e[i][1] + e[i][2] * e[i][2]);
+        g.s[i] = make_float4(e[i][0] / l, e[i][1] / l, e[i][2] / l, l);
+    }
+    // (b - a) x (c - a), c - a = -(a - c)
+    const float x = e[0][2] * e[2][1] - e[0][1] * e[2][2], y = e[0][0] * e[2][2] - e[0][2] * e[2][0],
+                z = e[0][1] * e[2][0] - e[0][0] * e[2][1];
+    const float nl = sqrtf(x * x + y * y + z * z);
+    g.n = nl > 0.0f ? make_float4(x / nl, y / nl, z / nl, nl) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    return g;
 }
 
 // P(x) = integral over the triangle of 1 / |x - y| dA and grad P(x), closed form (FP32; the
-// coordinates are taken relative to x so that near pairs keep their relative precision).
-__device__ void triangle_potential(const float x[3], const TriVerts &t, float &P, float G[3]) {
-    float a[3], b[3], c[3];
-    for (int k = 0; k < 3; k++) { a[k] = t.a[k] - x[k]; b[k] = t.b[k] - x[k]; c[k] = t.c[k] - x[k]; }
-    float e1[3], e2[3], n[3];
-    for (int k = 0; k < 3; k++) { e1[k] = b[k] - a[k]; e2[k] = c[k] - a[k]; }
-    n[0] = e1[1] * e2[2] - e1[2] * e2[1];
-    n[1] = e1[2] * e2[0] - e1[0] * e2[2];
-    n[2] = e1[0] * e2[1] - e1[1] * e2[0];
-    const float nl = sqrtf(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+// coordinates are taken relative to x so that near pairs keep their relative precision). Per edge the
+// logarithm ln((R+ + s+) / (R- + s-)), in the form without cancellation for the edge's side of the
+// projection; the three edges' arctangent terms add up to the triangle's solid angle, taken at once
+// (Van Oosterom and Strackee, IEEE Trans. Biomed. Eng. 30(2), 1983) instead of two arctangents and two
+// divisions per edge. With the geometry precomputed a pair costs some 200 instructions instead of 750.
+__device__ __forceinline__ void triangle_potential(const float x[3], const TriVerts &t, const TriGeom &g, float &P,
+                                                   float G[3]) {
+    float v[3][3];  // the vertices relative to x
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        v[0][k] = t.a[k] - x[k];
+        v[1][k] = t.b[k] - x[k];
+        v[2][k] = t.c[k] - x[k];
+    }
+    auto dot = [](const float *p, const float *q) { return p[0] * q[0] + p[1] * q[1] + p[2] * q[2]; };
+    const float n[3] = {g.n.x, g.n.y, g.n.z};
+    const float h = -dot(v[0], n), ah = fabsf(h);  // (x - a) . n with x at the origin
+    const float R[3] = {sqrtf(dot(v[0], v[0])), sqrtf(dot(v[1], v[1])), sqrtf(dot(v[2], v[2]))};
     P = 0.0f;
     G[0] = G[1] = G[2] = 0.0f;
-    if (!(nl > 0.0f)) return;
-    for (int k = 0; k < 3; k++) n[k] /= nl;
-    const float h = -(a[0] * n[0] + a[1] * n[1] + a[2] * n[2]);  // (x - a) . n with x at the origin
-    const float ah = fabsf(h);
-    float rho[3];
-    for (int k = 0; k < 3; k++) rho[k] = -h * n[k];
-    const float *vs[4] = {a, b, c, a};
-    float beta_sum = 0.0f;
+#pragma unroll
     for (int e = 0; e < 3; e++) {
-        const float *p0 = vs[e], *p1 = vs[e + 1];
-        float sv[3], m[3];
-        for (int k = 0; k < 3; k++) sv[k] = p1[k] - p0[k];
-        const float sl = sqrtf(sv[0] * sv[0] + sv[1] * sv[1] + sv[2] * sv[2]);
-        for (int k = 0; k < 3; k++) sv[k] /= sl;
-        m[0] = sv[1] * n[2] - sv[2] * n[1];
-        m[1] = sv[2] * n[0] - sv[0] * n[2];
-        m[2] = sv[0] * n[1] - sv[1] * n[0];
-        float sm = 0.0f, sp = 0.0f, tt = 0.0f, Rm2 = 0.0f, Rp2 = 0.0f;
-        for (int k = 0; k < 3; k++) {
-            sm += (p0[k] - rho[k]) * sv[k];
-            sp += (p1[k] - rho[k]) * sv[k];
-            tt += (p0[k] - rho[k]) * m[k];
-            Rm2 += p0[k] * p0[k];
-            Rp2 += p1[k] * p1[k];
-        }
-        const float R0sq = tt * tt + h * h;
-        if (!(R0sq > 0.0f)) continue;  // x on the edge's line: no contribution from this edge
-        const float Rm = sqrtf(Rm2), Rp = sqrtf(Rp2);
-        const float f = edge_log(Rp, sp, Rm, sm);
-        const float beta = atanf(tt * sp / (R0sq + ah * Rp)) - atanf(tt * sm / (R0sq + ah * Rm));
-        P += tt * f - ah * beta;
+        const float sv[3] = {g.s[e].x, g.s[e].y, g.s[e].z};
+        const float m[3] = {sv[1] * n[2] - sv[2] * n[1], sv[2] * n[0] - sv[0] * n[2], sv[0] * n[1] - sv[1] * n[0]};
+        const float sm = dot(v[e], sv), sp = sm + g.s[e].w, tt = dot(v[e], m);
+        const float Rm = R[e], Rp = R[(e + 1) % 3];
+        const bool ahead = sm + sp >= 0.0f;
+        const float num = ahead ? Rp + sp : Rm - sm, den = ahead ? Rm + sm : Rp - sp;
+        // x on the edge's line: no contribution from this edge
+        const float f = tt * tt + h * h > 0.0f ? logf(num / den) : 0.0f;
+        P += tt * f;
+#pragma unroll
         for (int k = 0; k < 3; k++) G[k] -= m[k] * f;
-        beta_sum += beta;
     }
-    const float sg = h > 0.0f ? 1.0f : (h < 0.0f ? -1.0f : 0.0f);
-    for (int k = 0; k < 3; k++) G[k] -= sg * beta_sum * n[k];
+    const float den = R[0] * R[1] * R[2] + dot(v[0], v[1]) * R[2] + dot(v[1], v[2]) * R[0] + dot(v[2], v[0]) * R[1];
+    const float omega = 2.0f * atan2f(ah * g.n.w, den);
+    P -= ah * omega;
+    const float sg = h > 0.0f ? omega : (h < 0.0f ? -omega : 0.0f);
+#pragma unroll
+    for (int k = 0; k < 3; k++) G[k] -= sg * n[k];
 }
 
 __device__ __forceinline__ void centroid_of(const TriVerts &t, float c[3]) {
     for (int k = 0; k < 3; k++) c[k] = (t.a[k] + t.b[k] + t.c[k]) / 3.0f;
 }
 
-// Per stored triangle: {centroid, sigma~ * area} and the squared near radius.
+// Per stored triangle: {centroid, sigma~ * area}, the squared near radius and the closed form's geometry.
 __global__ void cv_sources_kernel(SceneView<3> s, const float *__restrict__ sigma, float near_factor,
-                                  float4 *__restrict__ src, float *__restrict__ near2) {
+                                  float4 *__restrict__ src, float *__restrict__ near2, float4 *__restrict__ geom) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.n_elems) return;
     const TriVerts t = load_tri(s, i);
@@ -147,6 +158,9 @@ __global__ void cv_sources_kernel(SceneView<3> s, const float *__restrict__ sigm
     }
     src[i] = make_float4(c[0], c[1], c[2], sigma[i] * area);
     near2[i] = near_factor * near_factor * h2;
+    const TriGeom g = triangle_geometry(t);
+    geom[4 * (size_t)i] = g.n;
+    for (int e = 0; e < 3; e++) geom[4 * (size_t)i + 1 + e] = g.s[e];
 }
 
 constexpr int kClusterSize = 32;
@@ -211,7 +225,7 @@ __global__ void pts_morton_kernel(const float *__restrict__ pts, uint32_t n, uin
     key[i] = ((uint64_t)code << 32) | i;
 }
 // One warp per cluster: the record {z, r_far}, {M0, M1}, {M2xx, M2yy, M2zz, M2xy}, {M2xz, M2yz,
-// trace M2, 0}; r_far = max(rho / theta, rho + eta), infinite for theta = 0.
+// trace M2, rho + eta}; r_far = max(rho / theta, rho + eta), infinite for theta = 0.
 __global__ void cv_cluster_kernel(uint32_t n, const float4 *__restrict__ src, const float *__restrict__ near2,
                                   float theta, float4 *__restrict__ cl) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -237,7 +251,7 @@ __global__ void cv_cluster_kernel(uint32_t n, const float4 *__restrict__ src, co
         cl[4 * k + 0] = make_float4(zx, zy, zz, r_far);
         cl[4 * k + 1] = make_float4(m0, m1x, m1y, m1z);
         cl[4 * k + 2] = make_float4(mxx, myy, mzz, mxy);
-        cl[4 * k + 3] = make_float4(mxz, myz, mxx + myy + mzz, 0.0f);
+        cl[4 * k + 3] = make_float4(mxz, myz, mxx + myy + mzz, rho + eta);
     }
 }
 
@@ -318,18 +332,27 @@ __device__ __forceinline__ void cluster_field(const float x[3], const float4 &q0
 }
 
 // kMode 0: residual data at the stored triangles' centroids; kMode 1: potential and gradient at
-// points (out: [n][4] = u, du/dx, du/dy, du/dz). A block takes 32 consecutive targets (one per
-// lane); its kCvWarps warps split the cluster table (warp w takes clusters w, w + kCvWarps, ...)
-// and their sums are added in warp order through shared memory at the end.
+// points (out: [n][4] = u, du/dx, du/dy, du/dz).
+constexpr uint32_t kItems = 32 * kGroupFan * kGroupFan;  // clusters of a batch: far and near records together
+constexpr uint32_t kCheckNear = 0x80000000u;
+static_assert(32 * kGroupFan == kCvBlock, "a thread per middle group of a batch");
 template <int kMode>
-__global__ void __launch_bounds__(kCvBlock) cv_sum_kernel(SceneView<3> s, const float4 *__restrict__ src,
+__global__ void __launch_bounds__(kCvBlock, 4) cv_sum_kernel(SceneView<3> s, const float4 *__restrict__ src,
                                                           const float *__restrict__ near2,
+                                                          const float4 *__restrict__ geom,
                                                           const float *__restrict__ sigma,
                                                           const float4 *__restrict__ cl, const float *__restrict__ pts,
                                                           const uint64_t *__restrict__ order, uint32_t n_targets,
                                                           float c_coef, float *__restrict__ out,
                                                           double *__restrict__ part_sums) {
     __shared__ double s_acc[kCvWarps][4][32];
+    // triangles within some target's near radius, found by each warp in its order and, once all are
+    // found, dealt to the warps in turn: a block's closed forms sit in the few clusters around its
+    // targets, and the warps that met them kept the others waiting
+    __shared__ uint32_t s_near[kCvWarps][kNearList];
+    __shared__ uint32_t s_count[kCvWarps];
+    __shared__ uint32_t s_items[kItems], s_open[32 * kGroupFan], s_tally[kCvWarps];
+    uint32_t n_near = 0;
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint32_t slot = blockIdx.x * 32u + lane;
     const bool active = slot < n_targets;
@@ -357,7 +380,6 @@ __global__ void __launch_bounds__(kCvBlock) cv_sum_kernel(SceneView<3> s, const 
     float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     const uint32_t n_src = s.n_elems;
     const uint32_t n_cl = div_up(n_src, kClusterSize), n_g1 = div_up(n_cl, kGroupFan), n_g2 = div_up(n_g1, kGroupFan);
-    const float4 *g1 = cl + 4 * (size_t)n_cl, *g2 = g1 + 4 * (size_t)n_g1;
     uint32_t taken = 0;
     // far from every target of the block: |W - z| > r_far + omega
     auto is_far = [&](const float4 &q0) {
@@ -366,8 +388,8 @@ __global__ void __launch_bounds__(kCvBlock) cv_sum_kernel(SceneView<3> s, const 
         return Dx * Dx + Dy * Dy + Dz * Dz > thr * thr;
     };
     // a record's expansion at this lane's target; FP32 partial sums flushed to FP64 every 32 items
-    auto expand = [&](const float4 *r, const float4 &q0) {
-        const float4 q1 = __ldg(r + 1), q2 = __ldg(r + 2), q3 = __ldg(r + 3);
+    auto expand = [&](const float4 *r) {
+        const float4 q0 = __ldg(r), q1 = __ldg(r + 1), q2 = __ldg(r + 2), q3 = __ldg(r + 3);
         float phi, g[3];
         cluster_field(xd, q0, q1, q2, q3, phi, g);
         if (kMode == 0) {
@@ -382,82 +404,149 @@ __global__ void __launch_bounds__(kCvBlock) cv_sum_kernel(SceneView<3> s, const 
     auto flush = [&]() {
         if ((++taken & 31u) == 0u) {
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
+            for (int c = 0; c < (kMode == 0 ? 1 : 4); c++) {
                 acc[c] += a[c];
                 a[c] = 0.0f;
             }
         }
     };
-    // Every warp walks the same decisions (uniform across the block); the work is dealt by index:
-    // a far group or level-1 group to warp (index mod 8), the clusters of a near level-1 group one
-    // per warp, so the near field spreads over the warps as in a flat pass over the clusters.
-    // the largest groups are split over gridDim.y blocks of the same targets (part blockIdx.y takes
-    // k2 = part, part + gridDim.y, ...), whose sums part_sums holds for cv_parts_kernel
-    for (uint32_t k2 = blockIdx.y; k2 < n_g2; k2 += gridDim.y) {
-        const float4 h2 = __ldg(g2 + 4 * k2);
-        if (is_far(h2)) {
-            if (k2 % kCvWarps == wid) {
-                expand(g2 + 4 * k2, h2);
-                flush();
-            }
-            continue;
+    // triangle i's closed form at this lane's target where it is near
+    auto closed_form = [&](uint32_t i, bool near) {
+        if (!near || !active || (kMode == 0 && i == tgt)) return;
+        const float4 *q = geom + 4 * (size_t)i;
+        TriGeom g;
+        g.n = __ldg(q);
+        if (!(g.n.w > 0.0f)) return;
+        for (int e = 0; e < 3; e++) g.s[e] = __ldg(q + 1 + e);
+        float P, G[3];
+        triangle_potential(xd, load_tri(s, i), g, P, G);
+        const float sg = __ldg(sigma + i);
+        if (kMode == 0) {
+            a[0] -= sg * (G[0] * nn[0] + G[1] * nn[1] + G[2] * nn[2]);
+        } else {
+            a[0] += sg * P;
+            a[1] += sg * G[0];
+            a[2] += sg * G[1];
+            a[3] += sg * G[2];
         }
-        const uint32_t k1_end = min(n_g1, (k2 + 1) * kGroupFan);
-        for (uint32_t k1 = k2 * kGroupFan; k1 < k1_end; k1++) {
-            const float4 h1 = __ldg(g1 + 4 * k1);
-            if (is_far(h1)) {
-                if (k1 % kCvWarps == wid) {
-                    expand(g1 + 4 * k1, h1);
-                    flush();
-                }
-                continue;
+    };
+    // a source by the centroid rule (0 where `near`)
+    auto centroid_rule = [&](const float4 &q, float dx, float dy, float dz, float r2, bool near) {
+        const float rinv = near ? 0.0f : rsqrtf(r2);
+        const float r3 = rinv * rinv * rinv;
+        if (kMode == 0) {
+            a[0] += q.w * (dx * nn[0] + dy * nn[1] + dz * nn[2]) * r3;
+        } else {
+            a[0] += q.w * rinv;
+            const float wr3 = q.w * r3;
+            a[1] -= wr3 * dx;
+            a[2] -= wr3 * dy;
+            a[3] -= wr3 * dz;
+        }
+    };
+    // The records are decided a thread each, in batches of 32 largest groups (at most 2048 clusters): far
+    // ones are listed from the front of s_items, near clusters from its back, in a fixed order, and the
+    // warps then take the two lists in turn. Deciding in every warp, all lanes alike, was a sixth of the
+    // instructions, and dealing by index left the warps unevenly loaded. The largest groups are also
+    // split over gridDim.y blocks of the same targets (part blockIdx.y takes k2 = part, part +
+    // gridDim.y, ...), whose sums part_sums holds for cv_parts_kernel.
+    uint32_t n_far = 0, n_cls = 0;  // the lists' lengths (the same in every thread)
+    // appends `item` of the threads with `far` / `cls`, in thread order
+    auto append = [&](bool far, bool cls, uint32_t item) {
+        const uint32_t bf = __ballot_sync(0xffffffffu, far), bc = __ballot_sync(0xffffffffu, cls);
+        if (lane == 0) s_tally[wid] = (uint32_t)__popc(bf) | ((uint32_t)__popc(bc) << 16);
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kCvWarps; w++) {
+            const uint32_t c = s_tally[w];
+            if (w < wid) before += c;
+            all += c;
+        }
+        const uint32_t lt = (1u << lane) - 1u;
+        if (far) s_items[n_far + (before & 0xffffu) + (uint32_t)__popc(bf & lt)] = item;
+        if (cls) s_items[kItems - 1u - (n_cls + (before >> 16) + (uint32_t)__popc(bc & lt))] = item;
+        n_far += all & 0xffffu;
+        n_cls += all >> 16;
+        __syncthreads();
+    };
+    for (uint32_t b0 = blockIdx.y; b0 < n_g2; b0 += 32u * gridDim.y) {
+        n_far = n_cls = 0;
+        // the largest groups; near ones are opened (kept as the block's near list for a moment)
+        const uint32_t k2 = b0 + threadIdx.x * gridDim.y;
+        const bool in2 = threadIdx.x < 32u && k2 < n_g2;
+        const bool far2 = in2 && is_far(__ldg(cl + 4 * (size_t)(n_cl + n_g1 + k2)));
+        append(far2, in2 && !far2, far2 ? n_cl + n_g1 + k2 : k2);
+        const uint32_t open2 = n_cls;
+        const uint32_t slot1 = threadIdx.x / kGroupFan;
+        const uint32_t k1 = slot1 < open2 ? s_items[kItems - 1u - slot1] * kGroupFan + threadIdx.x % kGroupFan : n_g1;
+        const bool in1 = k1 < n_g1, far1 = in1 && is_far(__ldg(cl + 4 * (size_t)(n_cl + k1)));
+        __syncthreads();
+        n_cls = 0;
+        append(far1, in1 && !far1, far1 ? n_cl + k1 : k1);
+        const uint32_t open1 = n_cls;
+        if (threadIdx.x < open1) s_open[threadIdx.x] = s_items[kItems - 1u - threadIdx.x];
+        __syncthreads();
+        n_cls = 0;
+        for (uint32_t t0 = 0; t0 < open1 * kGroupFan; t0 += kCvBlock) {
+            const uint32_t slot = (t0 + threadIdx.x) / kGroupFan;
+            const uint32_t k = slot < open1 ? s_open[slot] * kGroupFan + threadIdx.x % kGroupFan : n_cl;
+            bool far = false, check = false;
+            if (k < n_cl) {
+                const float4 q0 = __ldg(cl + 4 * (size_t)k);
+                far = is_far(q0);
+                // can a member lie within a near radius of a target? (rounded towards yes)
+                const float Dx = Wx - q0.x, Dy = Wy - q0.y, Dz = Wz - q0.z;
+                const float reach = (__ldg(cl + 4 * (size_t)k + 3).w + om) * 1.00001f;
+                check = !(Dx * Dx + Dy * Dy + Dz * Dz > reach * reach);
             }
-            const uint32_t k_end = min(n_cl, (k1 + 1) * kGroupFan);
-            for (uint32_t k = k1 * kGroupFan + wid; k < k_end; k += kCvWarps) {
-                const float4 q0 = __ldg(cl + 4 * k);
-                if (is_far(q0)) {
-                    expand(cl + 4 * k, q0);
-                } else {
-                    const uint32_t i0 = k * kClusterSize, i1 = min(n_src, i0 + kClusterSize);
-                    for (uint32_t i = i0; i < i1; i++) {
-                        const float4 q = __ldg(src + i);
-                        const float n2 = __ldg(near2 + i);
-                        const float dx = xd[0] - q.x, dy = xd[1] - q.y, dz = xd[2] - q.z;
-                        const float r2 = dx * dx + dy * dy + dz * dz;
-                        const bool near = r2 < n2;
-                        if (!near) {
-                            const float rinv = rsqrtf(r2);
-                            const float r3 = rinv * rinv * rinv;
-                            if (kMode == 0) {
-                                a[0] += q.w * (dx * nn[0] + dy * nn[1] + dz * nn[2]) * r3;
-                            } else {
-                                a[0] += q.w * rinv;
-                                const float wr3 = q.w * r3;
-                                a[1] -= wr3 * dx;
-                                a[2] -= wr3 * dy;
-                                a[3] -= wr3 * dz;
-                            }
-                        }
-                        if (__any_sync(0xffffffffu, near && active)) {
-                            if (near && active && !(kMode == 0 && i == tgt)) {
-                                const TriVerts tri = load_tri(s, i);
-                                float P, G[3];
-                                triangle_potential(xd, tri, P, G);
-                                const float sg = __ldg(sigma + i);
-                                if (kMode == 0) {
-                                    a[0] -= sg * (G[0] * nn[0] + G[1] * nn[1] + G[2] * nn[2]);
-                                } else {
-                                    a[0] += sg * P;
-                                    a[1] += sg * G[0];
-                                    a[2] += sg * G[1];
-                                    a[3] += sg * G[2];
-                                }
-                            }
+            append(far, k < n_cl && !far, k | (check && !far ? kCheckNear : 0u));
+        }
+        for (uint32_t e = wid; e < n_far; e += kCvWarps) {
+            expand(cl + 4 * (size_t)s_items[e]);
+            flush();
+        }
+        for (uint32_t e = wid; e < n_cls; e += kCvWarps) {
+            const uint32_t item = s_items[kItems - 1u - e], k = item & ~kCheckNear;
+            const uint32_t i0 = k * kClusterSize, i1 = min(n_src, i0 + kClusterSize);
+            if (item & kCheckNear) {
+                for (uint32_t i = i0; i < i1; i++) {
+                    const float4 q = __ldg(src + i);
+                    const float dx = xd[0] - q.x, dy = xd[1] - q.y, dz = xd[2] - q.z;
+                    const float r2 = dx * dx + dy * dy + dz * dz;
+                    const bool near = r2 < __ldg(near2 + i);
+                    centroid_rule(q, dx, dy, dz, r2, near);
+                    if (__any_sync(0xffffffffu, near && active)) {
+                        if (n_near < kNearList) {
+                            if (lane == 0) s_near[wid][n_near] = i;
+                            n_near++;
+                        } else {
+                            closed_form(i, near);
                         }
                     }
                 }
-                flush();
+            } else {
+#pragma unroll 4
+                for (uint32_t i = i0; i < i1; i++) {
+                    const float4 q = __ldg(src + i);
+                    const float dx = xd[0] - q.x, dy = xd[1] - q.y, dz = xd[2] - q.z;
+                    centroid_rule(q, dx, dy, dz, dx * dx + dy * dy + dz * dz, false);
+                }
             }
+            flush();
+        }
+        __syncthreads();  // the lists are rebuilt by the next batch
+    }
+    if (lane == 0) s_count[wid] = n_near;
+    __syncthreads();
+    uint32_t at = wid;  // entry of the lists laid end to end
+    for (uint32_t w = 0, base = 0; w < kCvWarps; base += s_count[w], w++) {
+        for (; at < base + s_count[w]; at += kCvWarps) {
+            const uint32_t i = s_near[w][at - base];
+            const float4 q = __ldg(src + i);
+            const float dx = xd[0] - q.x, dy = xd[1] - q.y, dz = xd[2] - q.z;
+            closed_form(i, dx * dx + dy * dy + dz * dz < __ldg(near2 + i));
+            flush();
         }
     }
 #pragma unroll
@@ -530,8 +619,8 @@ template cudaError_t launch_element_frames<2>(const SceneView<2> &, float *, cud
 template cudaError_t launch_element_frames<3>(const SceneView<3> &, float *, cudaStream_t);
 
 cudaError_t launch_cv_sources(const SceneView<3> &s, const float *sigma, float near_factor, float theta, float4 *src,
-                              float *near2, float4 *clusters, cudaStream_t stream) {
-    cv_sources_kernel<<<(s.n_elems + 255) / 256, 256, 0, stream>>>(s, sigma, near_factor, src, near2);
+                              float *near2, float4 *geom, float4 *clusters, cudaStream_t stream) {
+    cv_sources_kernel<<<(s.n_elems + 255) / 256, 256, 0, stream>>>(s, sigma, near_factor, src, near2, geom);
     const uint32_t n_cl = div_up(s.n_elems, kClusterSize), n_g1 = div_up(n_cl, kGroupFan), n_g2 = div_up(n_g1, kGroupFan);
     cv_cluster_kernel<<<(n_cl * 32 + 255) / 256, 256, 0, stream>>>(s.n_elems, src, near2, theta, clusters);
     cv_group_kernel<kClusterSize * kGroupFan><<<n_g1, kGroupBlock, 0, stream>>>(s.n_elems, src, near2, theta,
@@ -546,9 +635,10 @@ uint32_t cv_cluster_records(uint32_t n_elems) {
     return n_cl + n_g1 + div_up(n_g1, kGroupFan);
 }
 
-cudaError_t launch_cv_residual(const SceneView<3> &s, const float4 *src, const float *near2, const float4 *clusters,
+cudaError_t launch_cv_residual(const SceneView<3> &s, const float4 *src, const float *near2, const float4 *geom,
+                               const float4 *clusters,
                                const float *sigma, float c_coef, float *delta, cudaStream_t stream) {
-    cv_sum_kernel<0><<<(s.n_elems + 31) / 32, kCvBlock, 0, stream>>>(s, src, near2, sigma, clusters, nullptr, nullptr,
+    cv_sum_kernel<0><<<(s.n_elems + 31) / 32, kCvBlock, 0, stream>>>(s, src, near2, geom, sigma, clusters, nullptr, nullptr,
                                                                      s.n_elems, c_coef, delta, nullptr);
     return cudaGetLastError();
 }
@@ -559,7 +649,8 @@ uint32_t cv_point_order_words(uint32_t n_points) {
     return 2 * n2 + 8 + kPotentialParts * n_points * 8;
 }
 
-cudaError_t launch_cv_potential(const SceneView<3> &s, const float4 *src, const float *near2, const float4 *clusters,
+cudaError_t launch_cv_potential(const SceneView<3> &s, const float4 *src, const float *near2, const float4 *geom,
+                                const float4 *clusters,
                                 const float *sigma, const float *pts, uint32_t n_points, uint32_t *scratch,
                                 float *out, cudaStream_t stream) {
     if (n_points == 0) return cudaSuccess;
@@ -573,7 +664,7 @@ cudaError_t launch_cv_potential(const SceneView<3> &s, const float4 *src, const 
     if (e != cudaSuccess) return e;
     double *part_sums = reinterpret_cast<double *>(scratch + 2 * (size_t)n2 + 8);
     cv_sum_kernel<1><<<dim3((n_points + 31) / 32, kPotentialParts), kCvBlock, 0, stream>>>(
-        s, src, near2, sigma, clusters, pts, key, n_points, 0.0f, out, part_sums);
+        s, src, near2, geom, sigma, clusters, pts, key, n_points, 0.0f, out, part_sums);
     cv_parts_kernel<<<(n_points + 255) / 256, 256, 0, stream>>>(part_sums, kPotentialParts, key, n_points, out);
     return cudaGetLastError();
 }
