@@ -126,11 +126,15 @@ __global__ void __launch_bounds__(kWalkBlock) wave_start_kernel(SceneView<3> s, 
 // instead of four). Each child's box is stored as 8-bit offsets on a power-of-two grid over the
 // node's own box: words 0-2 the node box's lower corner o (float), word 3 the grid's biased
 // exponents per axis (byte a), words 4-7 the children, words 8-13 the quantized bounds (word 8 + a:
-// lower bound on axis a, byte k for child k; word 11 + a: upper bounds), words 14-15 zero. Lower
-// bounds are rounded down and upper bounds up (in double), so every decoded box contains its
-// child's padded box up to one float rounding of o + q 2^e -- far inside the boxes' 1e-5 padding:
-// the box test stays conservative and the hits (decided by the exact triangle test) are unchanged.
+// lower bound on axis a, byte k for child k; word 11 + a: upper bounds), word 14 the mask of the
+// children in use, word 15 zero. A child node whose children are leaves of at most kMergedLeaf elements
+// together becomes one leaf over them (a leaf's elements are consecutive, so the hits and their order
+// stay): the median splits leave such two-leaf nodes at the bottom of most trees. Lower
+// bounds are rounded down and upper bounds up (in double) and by one step more, so every decoded box
+// contains its child's padded box with a grid step to spare, far more than the roundings of the
+// test: it stays conservative and the hits (decided by the exact triangle test) are unchanged.
 constexpr int kQNodeWords = 16;
+constexpr uint32_t kMergedLeaf = 6;  // at most 8, the leaf code's range
 
 __global__ void compress_nodes_kernel(const float4 *__restrict__ soa, uint32_t n_nodes, uint32_t *__restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -147,21 +151,23 @@ __global__ void compress_nodes_kernel(const float4 *__restrict__ soa, uint32_t n
             mx = fmax(mx, (double)q[12 + 4 * a + k]);
         }
         if (mn > mx) mn = mx = 0.0;
-        const float o = (float)mn <= mn ? (float)mn : nextafterf((float)mn, -INFINITY);  // o <= every lower bound
-        lo[a] = (double)o;
-        ext[a] = mx - lo[a];
+        ext[a] = mx - mn;
         int e = 0;
-        frexp(ext[a] / 255.0, &e);  // 2^e > ext / 255: 255 steps of 2^e cover the box
-        if (ext[a] <= 0.0) e = -126;
-        e = e < -126 ? -126 : (e > 127 ? 127 : e);
+        // 2^e > ext / 251: 255 steps of 2^e cover the box, a step on each side and the corner's rounding
+        frexp(fmax(ext[a], fabs(mn) * 2.5e-4) / 251.0, &e);
+        if (ext[a] <= 0.0 && mn == 0.0) e = -126;
+        e = e < -100 ? -100 : (e > 127 ? 127 : e);
+        const double corner = mn - 1.5 * ldexp(1.0, e);
+        const float o = (float)corner;  // off by under half a step: |mn| 2^-24 < 2^e / 16
+        lo[a] = (double)o;
         w[a] = __float_as_uint(o);
         w[3] |= (uint32_t)(e + 127) << (8 * a);
         const double step = ldexp(1.0, e);
         for (int k = 0; k < 4; k++) {
             double ql = 0.0, qh = 0.0;
             if (c[k] != kChildEmptyD) {
-                ql = floor(((double)q[4 * a + k] - lo[a]) / step);
-                qh = ceil(((double)q[12 + 4 * a + k] - lo[a]) / step);
+                ql = floor(((double)q[4 * a + k] - lo[a]) / step) - 1.0;
+                qh = ceil(((double)q[12 + 4 * a + k] - lo[a]) / step) + 1.0;
             }
             ql = fmin(fmax(ql, 0.0), 255.0);
             qh = fmin(fmax(qh, 0.0), 255.0);
@@ -169,19 +175,52 @@ __global__ void compress_nodes_kernel(const float4 *__restrict__ soa, uint32_t n
             w[11 + a] |= (uint32_t)qh << (8 * k);
         }
     }
-    for (int k = 0; k < 4; k++) w[4 + k] = c[k];
+    for (int k = 0; k < 4; k++) {
+        uint32_t code = c[k];
+        if (code != kChildEmptyD) {
+            w[14] |= 1u << k;
+            if (!(code & 0x80000000u)) {
+                const uint32_t *g = reinterpret_cast<const uint32_t *>(soa + 8 * (size_t)code) + 24;
+                uint32_t first = 0xFFFFFFFFu, total = 0;
+                bool leaves = true;
+                for (int q4 = 0; q4 < 4; q4++) {
+                    if (g[q4] == kChildEmptyD) continue;
+                    if (!(g[q4] & 0x80000000u)) {
+                        leaves = false;
+                        break;
+                    }
+                    first = min(first, g[q4] & 0x0FFFFFFFu);
+                    total += ((g[q4] >> 28) & 7u) + 1u;
+                }
+                if (leaves && total > 0u && total <= kMergedLeaf) code = 0x80000000u | ((total - 1u) << 28) | first;
+            }
+        }
+        w[4 + k] = code;
+    }
     uint4 *dst = reinterpret_cast<uint4 *>(out + (size_t)i * kQNodeWords);
     for (int v = 0; v < 4; v++) dst[v] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
 }
 
 // The slab test against a compressed node's four children. With the node's corner o and grid step
 // s = 2^e per axis, a child bound o + q s lies on the line at t = q (s r) + (o r - O r): s r is exact
-// (a power of two times r), o r - O r one FMA per axis and node, and each bound then one FMA. q is
-// formed exactly by a byte permute into the float 2^23 + q and one subtraction, which keeps the
-// conversion off the special-function pipe. The t's rounding is of the order of the uncompressed
-// test's, far inside the boxes' padding.
+// (a power of two times r), o r - O r one FMA per axis and node. A byte permute forms the float
+// 2^15 + q, and 2^15 (s r) is taken off the node's constant instead of off every bound: that constant's
+// rounding moves a bound by at most some 2^-8 of a grid step, well inside the step the bounds keep in
+// reserve. The two bounds of a child and axis are one packed FMA (fma.rn.f32x2): 12 per node beside
+// 24 permutes, where converting and evaluating each bound took 72 instructions.
+__device__ __forceinline__ uint64_t pack_f2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void fma_f2(uint64_t x, uint64_t a, uint64_t b, float &lo, float &hi) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(r));
+}
+// 2^15 + byte k of the word
 __device__ __forceinline__ float qbyte(uint32_t word, uint32_t k) {
-    return __uint_as_float(__byte_perm(word, 0x4B000000u, 0x7540u + k)) - 8388608.0f;
+    return __uint_as_float(__byte_perm(word, 0x47000000u, 0x7604u + (k << 4)));
 }
 __device__ __forceinline__ uint32_t qnode_hits(const uint32_t *__restrict__ qn, uint32_t node, const LineSlab3 &L,
                                                uint4 &child) {
@@ -193,34 +232,42 @@ __device__ __forceinline__ uint32_t qnode_hits(const uint32_t *__restrict__ qn, 
                        __float_as_uint(r0.b.w));
     const uint32_t qlo[3] = {__float_as_uint(r1.a.x), __float_as_uint(r1.a.y), __float_as_uint(r1.a.z)};
     const uint32_t qhi[3] = {__float_as_uint(r1.a.w), __float_as_uint(r1.b.x), __float_as_uint(r1.b.y)};
-    float A[3], B[3];
+    uint64_t A[3], B[3];
+    uint32_t qn_[3], qf_[3];  // the bounds the line meets first and last, by the direction's sign
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        A[a] = __uint_as_float(((ex >> (8 * a)) & 0xFFu) << 23) * L.r[a];
-        B[a] = __fmaf_rn(o[a], L.r[a], L.nor[a]);
+        qn_[a] = L.r[a] < 0.0f ? qhi[a] : qlo[a];
+        qf_[a] = L.r[a] < 0.0f ? qlo[a] : qhi[a];
+        const float sa = __uint_as_float(((ex >> (8 * a)) & 0xFFu) << 23) * L.r[a];
+        const float ba = __fmaf_rn(-32768.0f, sa, __fmaf_rn(o[a], L.r[a], L.nor[a]));
+        A[a] = pack_f2(sa, sa);
+        B[a] = pack_f2(ba, ba);
     }
     uint32_t mask = 0;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         float tl[3], th[3];
 #pragma unroll
-        for (int a = 0; a < 3; a++) {
-            tl[a] = __fmaf_rn(qbyte(qlo[a], (uint32_t)k), A[a], B[a]);
-            th[a] = __fmaf_rn(qbyte(qhi[a], (uint32_t)k), A[a], B[a]);
-        }
-        const float tn = fmax3f(fminf(tl[0], th[0]), fminf(tl[1], th[1]), fminf(tl[2], th[2]));
-        const float tf = fmin3f(fmaxf(tl[0], th[0]), fmaxf(tl[1], th[1]), fmaxf(tl[2], th[2]));
-        if (tn <= tf) mask |= 1u << k;
+        for (int a = 0; a < 3; a++)
+            fma_f2(pack_f2(qbyte(qn_[a], (uint32_t)k), qbyte(qf_[a], (uint32_t)k)), A[a], B[a], tl[a], th[a]);
+        if (fmax3f(tl[0], tl[1], tl[2]) <= fmin3f(th[0], th[1], th[2])) mask |= 1u << k;
     }
-    return mask;
+    return mask & __float_as_uint(r1.b.z);
 }
 
-// The trace phase. kLeaves: leaves a lane holds before testing them (line_query3's kLeafBatch);
-// kQuant: node visits read the compressed nodes (qnodes) instead of the scene's.
+// The trace phase. kLeaves: leaves a lane holds at most; kQuant: node visits read the compressed nodes
+// (qnodes) instead of the scene's.
+//
+// A lane's query is in up to two states at once -- an inner node to visit, leaves held for testing -- or
+// finished, and each iteration the warp executes the step that most of its lanes can take: a node
+// visit, the test of one held leaf, or the choice of the hit and the fetch of the next query.
+// Descending in every lane until its leaves were held, then testing them all, kept 11.5 of 32 lanes
+// active (ALU pipe 66 %: issue-bound), because both loops run as long as their longest lane. Leaves
+// queue in the order they are met, so the hits keep their order.
 template <int kMinB, int kLeaves, bool kQuant>
 __global__ void __launch_bounds__(kWalkBlock, kMinB) wave_trace_kernel(SceneView<3> s, WalkParams p, WaveArgs a,
                                                                       const uint32_t *__restrict__ qnodes) {
-    static_assert(kLeaves <= kLeafBatch, "leaf columns hold kLeafBatch entries");
+    static_assert(kLeaves <= kLeafBatch && (kLeaves & (kLeaves - 1)) == 0, "leaf columns hold kLeafBatch entries, a ring");
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t *const my_stack = stack_column();
     uint32_t *const my_leaf = leaf_column();
@@ -230,19 +277,116 @@ __global__ void __launch_bounds__(kWalkBlock, kMinB) wave_trace_kernel(SceneView
     V<3> o, d;
     uint32_t j = 0, code = 0, steps = 0, count = 0;
     int sp = 0;
-    bool busy = false, fetch = true;
+    uint32_t held = 0, head = 0;           // leaves held: ring entries [head, head + held)
+    bool busy = false, live = false;       // a query assigned; its traversal unfinished
+    bool fetch = true;
+    // From `code`, the next one of the traversal: leaves go to the ring while it has room; stops at an
+    // inner node, a leaf that has to wait, or the end of the traversal.
+    auto advance = [&]() {
+        while (live && (code & 0x80000000u) && held < (uint32_t)kLeaves) {
+            if (++steps > s.traversal_limit) {
+                atomicOr(s.err, kErrTraversalLimit);
+                live = false;
+                break;
+            }
+            my_leaf[((head + held) & (kLeaves - 1u)) * kWalkBlock] = code;
+            held++;
+            if (sp == 0) {
+                live = false;
+                break;
+            }
+            sp--;
+            code = sp < kSharedStack ? my_stack[sp * kWalkBlock] : spill[sp - kSharedStack];
+        }
+    };
     while (true) {
-        // lanes without a query take the next slots: one atomic for the warp
-        const uint32_t need = __ballot_sync(kFull, fetch);
-        if (need) {
+        const bool node = live && !(code & 0x80000000u);
+        const int n_node = __popc(__ballot_sync(kFull, node));
+        const int n_leaf = __popc(__ballot_sync(kFull, held != 0u));
+        const bool done = busy && !live && held == 0u;
+        const uint32_t need = __ballot_sync(kFull, fetch || done);
+        const int n_done = __popc(need);
+        if (n_node == 0 && n_leaf == 0 && n_done == 0) break;
+        if (n_node >= n_leaf && n_node >= n_done) {
+            if (node) {
+                if (++steps > s.traversal_limit) {
+                    atomicOr(s.err, kErrTraversalLimit);
+                    live = false;
+                } else {
+                    uint4 ch;
+                    uint32_t keep = kQuant ? qnode_hits(qnodes, code, L, ch) : node_hits(s, code, L, ch);
+                    const uint32_t cs[4] = {ch.x, ch.y, ch.z, ch.w};
+                    if constexpr (!kQuant) {
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            if (cs[k] == kChildEmptyD) keep &= ~(1u << k);
+                    }
+                    if (keep) {
+                        if (sp + 3 > (int)kStackSize) {
+                            atomicOr(s.err, kErrStackOverflow);
+                            live = false;
+                        } else {
+                            const uint32_t first = (uint32_t)(__ffs(keep) - 1);
+                            const uint32_t later = keep & (keep - 1u);
+                            if (__builtin_expect(sp + 3 <= kSharedStack, 1)) {
+                                uint32_t *top = my_stack + sp * kWalkBlock;
+#pragma unroll
+                                for (int k = 3; k >= 1; k--)
+                                    if ((later >> k) & 1u) {
+                                        *top = cs[k];
+                                        top += kWalkBlock;
+                                    }
+                                sp += __popc(later);
+                            } else {
+#pragma unroll
+                                for (int k = 3; k >= 1; k--)
+                                    if ((later >> k) & 1u) {
+                                        if (sp < kSharedStack) my_stack[sp * kWalkBlock] = cs[k];
+                                        else spill[sp - kSharedStack] = cs[k];
+                                        sp++;
+                                    }
+                            }
+                            code = first == 0u ? cs[0] : first == 1u ? cs[1] : first == 2u ? cs[2] : cs[3];
+                        }
+                    } else if (sp == 0) {
+                        live = false;
+                    } else {
+                        sp--;
+                        code = sp < kSharedStack ? my_stack[sp * kWalkBlock] : spill[sp - kSharedStack];
+                    }
+                    advance();
+                }
+            }
+        } else if (n_leaf >= n_done) {
+            if (held) {
+                const uint32_t leaf = my_leaf[(head & (kLeaves - 1u)) * kWalkBlock];
+                head++;
+                held--;
+                count = leaf_hits<3>(s, leaf, o, d, hits, count);
+                advance();
+            }
+        } else {
+            if (done) {
+                // the query is complete: choose the hit with the path's next draw
+                uint32_t pt, path;
+                slot_point(p, a, j, pt, path);
+                PathRng rng(p.seed, kStreamDomain, p.point_offset + pt, p.path_offset + path);
+                rng.seek(a.draws[j]);
+                uint32_t m = count;
+                a.hit[j] = line_hit_choice(rng, hits, m);
+                a.nhit[j] = m;
+                busy = false;
+                fetch = true;
+            }
+            // lanes without a query take the next slots: one atomic for the warp
             const int leader = __ffs(need) - 1;
             uint32_t base = 0;
-            if ((int)lane == leader) base = atomicAdd(a.counter, (uint32_t)__popc(need));
+            if ((int)lane == leader) base = atomicAdd(a.counter, (uint32_t)n_done);
             base = __shfl_sync(kFull, base, leader);
             if (fetch) {
                 j = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
                 fetch = false;
-                busy = j < a.n;
+                busy = live = j < a.n;
                 if (busy) {
 #pragma unroll
                     for (int i = 0; i < 3; i++) {
@@ -256,66 +400,6 @@ __global__ void __launch_bounds__(kWalkBlock, kMinB) wave_trace_kernel(SceneView
                     count = 0;
                 }
             }
-        }
-        if (!__any_sync(kFull, busy)) break;
-        if (!busy) continue;
-        // one round of line_query3: nodes until kLeaves leaves are held or the stack is empty,
-        // then the held leaves in the order they were met
-        int nl = 0;
-        bool live = true;
-        while (nl < kLeaves) {
-            if (++steps > s.traversal_limit) {
-                atomicOr(s.err, kErrTraversalLimit);
-                live = false;
-                break;
-            }
-            if (code & 0x80000000u) {
-                my_leaf[nl * kWalkBlock] = code;
-                nl++;
-            } else {
-                uint4 ch;
-                uint32_t keep = kQuant ? qnode_hits(qnodes, code, L, ch) : node_hits(s, code, L, ch);
-                const uint32_t cs[4] = {ch.x, ch.y, ch.z, ch.w};
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (cs[k] == kChildEmptyD) keep &= ~(1u << k);
-                if (keep) {
-                    if (sp + 3 > (int)kStackSize) {
-                        atomicOr(s.err, kErrStackOverflow);
-                        live = false;
-                        break;
-                    }
-                    const uint32_t first = (uint32_t)(__ffs(keep) - 1);
-#pragma unroll
-                    for (int k = 3; k >= 1; k--)
-                        if ((uint32_t)k > first && ((keep >> k) & 1u)) {
-                            if (sp < kSharedStack) my_stack[sp * kWalkBlock] = cs[k];
-                            else spill[sp - kSharedStack] = cs[k];
-                            sp++;
-                        }
-                    code = cs[first];
-                    continue;
-                }
-            }
-            if (sp == 0) {
-                live = false;
-                break;
-            }
-            sp--;
-            code = sp < kSharedStack ? my_stack[sp * kWalkBlock] : spill[sp - kSharedStack];
-        }
-        for (int l = 0; l < nl; l++) count = leaf_hits<3>(s, my_leaf[l * kWalkBlock], o, d, hits, count);
-        if (!live) {
-            // the query is complete: choose the hit with the path's next draw
-            uint32_t pt, path;
-            slot_point(p, a, j, pt, path);
-            PathRng rng(p.seed, kStreamDomain, p.point_offset + pt, p.path_offset + path);
-            rng.seek(a.draws[j]);
-            uint32_t m = count;
-            a.hit[j] = line_hit_choice(rng, hits, m);
-            a.nhit[j] = m;
-            busy = false;
-            fetch = true;
         }
     }
 }
