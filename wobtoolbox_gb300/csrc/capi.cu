@@ -12,6 +12,7 @@
 #include "vpl.hpp"
 #include "wos.hpp"
 #include "scene_host.hpp"
+#include "scratch.hpp"
 #include "walk_generic.cuh"
 
 #include <algorithm>
@@ -155,7 +156,15 @@ struct wob_scene_s {
         v.vol_size = vol_size;
         return v;
     }
-    ~wob_scene_s() { release_all(); }
+    bool counted = false;  // holds the device's scratch pool
+    void count() {
+        wobgb::scratch_retain(device);
+        counted = true;
+    }
+    ~wob_scene_s() {
+        release_all();
+        if (counted) wobgb::scratch_release(device);
+    }
     void release_all() {
         for (DevBuf *b : {&elems, &elem_aux, &isect, &nodes, &area_cdf, &area_guide, &bv_cdf, &bv_guide, &err, &vol_values,
                           &vol_cdf, &vol_guide, &cv_table, &rhs, &rhs_cv, &ws, &lg_bins, &lg_off, &lg_ent, &lg_seg})
@@ -363,6 +372,7 @@ static int scene_create_impl(int dim, uint32_t n_elems, const float *vertices, c
     }
     s->host.release_tables();
     s->host.host_built = true;
+    s->count();
     *out = owner.release();
     return WOB_OK;
 }
@@ -421,6 +431,7 @@ static int scene_create_device_impl(int dim, uint32_t n_elems, const float *vert
         s->release_all();
         return fail_cuda(e, "allocating the error word");
     }
+    s->count();
     *out = owner.release();
     return WOB_OK;
 }
@@ -556,10 +567,10 @@ static int solve_domain_host_impl(wob_scene s, const wob_params *params, const f
     if (!points || !sum) return fail(WOB_ERR_INVALID_ARGUMENT, "points and sum are required");
     const int D = s->host.dim;
     const size_t pts_bytes = (size_t)n_points * D * 4, out_bytes = (size_t)n_points * (D + 1) * 8;
-    const size_t off_sum = (pts_bytes + 255) / 256 * 256;
-    const size_t off_sq = off_sum + (out_bytes + 255) / 256 * 256;
-    const size_t off_b = off_sq + (out_bytes + 255) / 256 * 256;
-    const size_t total = off_b + 256;
+    // points | sums | squares | {bounces, error word}: one clear and one copy back
+    const size_t off_sum = align256(pts_bytes);
+    const size_t off_sq = off_sum + out_bytes, off_tail = off_sq + (sumsq ? out_bytes : 0);
+    const size_t total = off_tail + 16;
     std::lock_guard<std::mutex> lock(s->ws_mutex);
     DeviceGuard g(s->device);
     cudaError_t e;
@@ -573,35 +584,30 @@ static int solve_domain_host_impl(wob_scene s, const wob_params *params, const f
     char *base = (char *)s->ws.ptr;
     float *d_pts = (float *)base;
     double *d_sum = (double *)(base + off_sum);
-    double *d_sq = (double *)(base + off_sq);
-    uint64_t *d_b = (uint64_t *)(base + off_b);
+    double *d_sq = sumsq ? (double *)(base + off_sq) : nullptr;
+    uint64_t *d_tail = (uint64_t *)(base + off_tail);
     cudaStream_t st_ = s->ws_stream;
     if ((e = cudaMemcpyAsync(d_pts, points, pts_bytes, cudaMemcpyHostToDevice, st_)) != cudaSuccess ||
-        (e = cudaMemsetAsync(d_sum, 0, out_bytes, st_)) != cudaSuccess ||
-        (e = cudaMemsetAsync(d_sq, 0, out_bytes, st_)) != cudaSuccess ||
-        (e = cudaMemsetAsync(d_b, 0, 8, st_)) != cudaSuccess)
+        (e = cudaMemsetAsync(d_sum, 0, total - off_sum, st_)) != cudaSuccess)
         return fail_cuda(e, "staging inputs");
-    e = D == 2 ? wobgb::launch_domain_2d(s->view<2>(), w, d_pts, n_points, d_sum, sumsq ? d_sq : nullptr,
-                                         (unsigned long long *)d_b, nullptr, st_)
-               : wobgb::launch_domain_3d(s->view<3>(), w, d_pts, n_points, d_sum, sumsq ? d_sq : nullptr,
-                                         (unsigned long long *)d_b, nullptr, st_);
+    e = D == 2 ? wobgb::launch_domain_2d(s->view<2>(), w, d_pts, n_points, d_sum, d_sq, (unsigned long long *)d_tail,
+                                         nullptr, st_)
+               : wobgb::launch_domain_3d(s->view<3>(), w, d_pts, n_points, d_sum, d_sq, (unsigned long long *)d_tail,
+                                         nullptr, st_);
     if (e != cudaSuccess) return fail_cuda(e, "launching the domain walk");
-    std::vector<double> tmp((size_t)n_points * (D + 1));
-    uint64_t b = 0;
-    uint32_t errw = 0;
-    if ((e = cudaMemcpyAsync(tmp.data(), d_sum, out_bytes, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&b, d_b, 8, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&errw, s->err.ptr, 4, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
+    const size_t n_out = (size_t)n_points * (D + 1);
+    std::vector<uint64_t> back((total - off_sum) / 8);
+    if ((e = cudaMemcpyAsync(d_tail + 1, s->err.ptr, 4, cudaMemcpyDeviceToDevice, st_)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(back.data(), d_sum, total - off_sum, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st_)) != cudaSuccess)
         return fail_cuda(e, "reading results");
-    for (size_t i = 0; i < tmp.size(); i++) sum[i] += tmp[i];
-    if (sumsq) {
-        if ((e = cudaMemcpyAsync(tmp.data(), d_sq, out_bytes, cudaMemcpyDeviceToHost, st_)) != cudaSuccess ||
-            (e = cudaStreamSynchronize(st_)) != cudaSuccess)
-            return fail_cuda(e, "reading results");
-        for (size_t i = 0; i < tmp.size(); i++) sumsq[i] += tmp[i];
-    }
-    if (bounces) *bounces += b;
+    const double *got = (const double *)back.data();
+    for (size_t i = 0; i < n_out; i++) sum[i] += got[i];
+    if (sumsq)
+        for (size_t i = 0; i < n_out; i++) sumsq[i] += got[n_out + i];
+    const uint64_t *tail = back.data() + (off_tail - off_sum) / 8;
+    const uint32_t errw = (uint32_t)tail[1];
+    if (bounces) *bounces += tail[0];
     if (errw) return fail(WOB_ERR_DEVICE_LIMIT, "a BVH traversal hit its stack or step bound");
     return WOB_OK;
 }
@@ -997,6 +1003,7 @@ int scene_clone_impl(wob_scene src, wob_scene *out) {
         s->release_all();
         return fail_cuda(e, "allocating the error word");
     }
+    s->count();
     *out = owner.release();
     return WOB_OK;
 }
@@ -1009,7 +1016,7 @@ int scene_add_boundary_offsets_impl(wob_scene s, const float *delta, uint32_t n,
     cudaStream_t st = (cudaStream_t)stream;
     // everything on the device: the records' adds and the new |g| tables, in buffers that replace the
     // scene's once the offsets are known to be finite (a clone's source keeps the shared old ones)
-    DevBuf scratch, cdf, guide;
+    DevBuf cdf, guide;
     wobgb::HostScene &h = s->host;
     const uint32_t G = wobgb::guide_records(n);
     const size_t work = wobgb::offset_scratch_bytes(n);
@@ -1018,25 +1025,27 @@ int scene_add_boundary_offsets_impl(wob_scene s, const float *delta, uint32_t n,
         if (r == cudaSuccess) b.bytes = bytes;
         return r;
     };
+    void *scratch = nullptr;
     auto drop = [&] {
-        for (DevBuf *b : {&scratch, &cdf, &guide}) b->release();
+        for (DevBuf *b : {&cdf, &guide}) b->release();
+        wobgb::scratch_free(scratch, st);
     };
     wobgb::OffsetResult res{};
     const float *dd = delta;
     cudaError_t e;
-    if ((e = alloc(scratch, work + (on_device ? 0 : (size_t)n * 4))) != cudaSuccess ||
+    if ((e = wobgb::scratch_alloc(&scratch, work + (on_device ? 0 : (size_t)n * 4), st)) != cudaSuccess ||
         (e = alloc(cdf, (size_t)n * 4)) != cudaSuccess || (e = alloc(guide, (size_t)G * 16)) != cudaSuccess) {
         drop();
         return fail_cuda(e, "allocating the boundary value tables");
     }
     if (!on_device) {
-        dd = (const float *)((char *)scratch.ptr + work);
+        dd = (const float *)((char *)scratch + work);
         e = cudaMemcpyAsync((void *)dd, delta, (size_t)n * 4, cudaMemcpyHostToDevice, st);
     }
     if (e != cudaSuccess ||
         (e = wobgb::launch_boundary_offsets(h.dim, n, dd, (float *)s->elems.ptr, (const float4 *)s->elem_aux.ptr,
-                                            (float *)cdf.ptr, G, (uint32_t *)guide.ptr, scratch.ptr, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(&res, scratch.ptr, sizeof res, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+                                            (float *)cdf.ptr, G, (uint32_t *)guide.ptr, scratch, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&res, scratch, sizeof res, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess) {
         drop();
         return fail_cuda(e, "updating the boundary values");
@@ -1059,31 +1068,39 @@ int scene_add_boundary_offsets_impl(wob_scene s, const float *delta, uint32_t n,
         s->bv_G = 1u;
         e = upload(s->bv_guide, none, sizeof none);
     }
-    scratch.release();
+    wobgb::scratch_free(scratch, st);
     return e == cudaSuccess ? WOB_OK : fail_cuda(e, "updating the boundary values");
 }
 
-// Triangle sources and clusters of sigma~ in a scratch allocation freed on return.
+// Triangle sources and clusters of sigma~, and `extra` bytes more, in one scratch allocation.
 struct CvSources {
-    DevBuf src, near2, geom, clusters;
+    cudaStream_t st;
+    void *base = nullptr;
+    float4 *src = nullptr, *geom = nullptr, *clusters = nullptr;
+    float *near2 = nullptr;
+    void *extra = nullptr;
+    explicit CvSources(cudaStream_t s) : st(s) {}
+    ~CvSources() { wobgb::scratch_free(base, st); }
 };
-int cv_sources(wob_scene s, const float *sigma, float near_factor, float theta, CvSources &cs, cudaStream_t st) {
+int cv_sources(wob_scene s, const float *sigma, float near_factor, float theta, size_t extra, CvSources &cs) {
     if (s->host.dim != 3) return fail(WOB_ERR_UNSUPPORTED, "the control-variate tables are implemented for 3D scenes");
     if (!sigma) return fail(WOB_ERR_INVALID_ARGUMENT, "sigma is required");
     if (!(near_factor >= 0.0f) || !(near_factor < 1e6f)) return fail(WOB_ERR_INVALID_ARGUMENT, "near_factor must be in [0, 1e6)");
     if (!(theta >= 0.0f) || !(theta < 1.0f)) return fail(WOB_ERR_INVALID_ARGUMENT, "theta must be in [0, 1)");
     const size_t n = s->host.n;
     const size_t n_rec = wobgb::cv_cluster_records((uint32_t)n);  // clusters and their two group levels
-    cudaError_t e;
-    if ((e = cudaMalloc(&cs.src.ptr, n * 16)) != cudaSuccess || (e = cudaMalloc(&cs.near2.ptr, n * 4)) != cudaSuccess ||
-        (e = cudaMalloc(&cs.geom.ptr, n * 64)) != cudaSuccess ||
-        (e = cudaMalloc(&cs.clusters.ptr, n_rec * 64)) != cudaSuccess)
-        return fail_cuda(e, "allocating the control-variate sources");
-    cs.src.bytes = n * 16;
-    cs.near2.bytes = n * 4;
-    cs.clusters.bytes = n_rec * 64;
-    e = wobgb::launch_cv_sources(s->view<3>(), sigma, near_factor, theta, (float4 *)cs.src.ptr, (float *)cs.near2.ptr,
-                                 (float4 *)cs.geom.ptr, (float4 *)cs.clusters.ptr, st);
+    const size_t sizes[5] = {n * 16, n * 64, n_rec * 64, n * 4, extra};
+    size_t off[6] = {};
+    for (int k = 0; k < 5; k++) off[k + 1] = off[k] + align256(sizes[k]);
+    cudaError_t e = wobgb::scratch_alloc(&cs.base, off[5], cs.st);
+    if (e != cudaSuccess) return fail_cuda(e, "allocating the control-variate sources");
+    char *b = (char *)cs.base;
+    cs.src = (float4 *)(b + off[0]);
+    cs.geom = (float4 *)(b + off[1]);
+    cs.clusters = (float4 *)(b + off[2]);
+    cs.near2 = (float *)(b + off[3]);
+    cs.extra = b + off[4];
+    e = wobgb::launch_cv_sources(s->view<3>(), sigma, near_factor, theta, cs.src, cs.near2, cs.geom, cs.clusters, cs.st);
     return e == cudaSuccess ? WOB_OK : fail_cuda(e, "launching the control-variate sources");
 }
 }  // namespace
@@ -1156,21 +1173,15 @@ int wob_cv_residual_data(wob_scene s, const float *sigma, int domain, float near
             return fail(WOB_ERR_INVALID_ARGUMENT, "domain must be 0 (interior) or 1 (exterior)");
         DeviceGuard g(s->device);
         cudaStream_t st = (cudaStream_t)stream;
-        CvSources cs;
-        int r = cv_sources(s, sigma, near_factor, theta, cs, st);
+        CvSources cs(st);
+        int r = cv_sources(s, sigma, near_factor, theta, 0, cs);
         if (r == WOB_OK) {
             // c = domain_type_coefficient / integral_free_term(1/2) (bie_models.cuh:66-78)
             const float c = domain == WOB_INTERIOR_DOMAIN ? 2.0f : -2.0f;
-            cudaError_t e = wobgb::launch_cv_residual(s->view<3>(), (const float4 *)cs.src.ptr, (const float *)cs.near2.ptr,
-                                                      (const float4 *)cs.geom.ptr, (const float4 *)cs.clusters.ptr, sigma, c,
-                                                      delta, st);
+            cudaError_t e = wobgb::launch_cv_residual(s->view<3>(), cs.src, cs.near2, cs.geom, cs.clusters, sigma, c, delta, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) r = fail_cuda(e, "computing the residual data");
         }
-        cs.src.release();
-        cs.near2.release();
-        cs.geom.release();
-        cs.clusters.release();
         return r;
     });
 }
@@ -1183,27 +1194,14 @@ int wob_cv_potential(wob_scene s, const float *sigma, float near_factor, float t
         if (!points || !out) return fail(WOB_ERR_INVALID_ARGUMENT, "points and out are required");
         DeviceGuard g(s->device);
         cudaStream_t st = (cudaStream_t)stream;
-        CvSources cs;
-        DevBuf order;
-        int r = cv_sources(s, sigma, near_factor, theta, cs, st);
+        CvSources cs(st);
+        int r = cv_sources(s, sigma, near_factor, theta, (size_t)wobgb::cv_point_order_words(n_points) * 4, cs);
         if (r == WOB_OK) {
-            const size_t words = wobgb::cv_point_order_words(n_points);
-            cudaError_t e = cudaMalloc(&order.ptr, words * 4);
-            if (e == cudaSuccess) {
-                order.bytes = words * 4;
-                e = wobgb::launch_cv_potential(s->view<3>(), (const float4 *)cs.src.ptr, (const float *)cs.near2.ptr,
-                                               (const float4 *)cs.geom.ptr, (const float4 *)cs.clusters.ptr, sigma, points,
-                                               n_points,
-                                               (uint32_t *)order.ptr, out, st);
-            }
+            cudaError_t e = wobgb::launch_cv_potential(s->view<3>(), cs.src, cs.near2, cs.geom, cs.clusters, sigma, points,
+                                                       n_points, (uint32_t *)cs.extra, out, st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) r = fail_cuda(e, "computing the control-variate potential");
         }
-        cs.src.release();
-        cs.near2.release();
-        cs.geom.release();
-        cs.clusters.release();
-        order.release();
         return r;
     });
 }

@@ -23,6 +23,7 @@
 // over a point's paths differs. Path state lives in HBM between phases (about 84 bytes a path,
 // structure of arrays, coalesced), in chunks of whole points.
 #include "kernels.cuh"
+#include "scratch.hpp"
 
 namespace wobgb {
 
@@ -510,7 +511,7 @@ cudaError_t launch_fwd_wave_3d(const SceneView<3> &s, const WalkParams &p, const
     const size_t q_off = (words * 4 + 255) / 256 * 256;  // bytes; the compressed nodes 256-byte aligned
     const size_t bytes = q_off + (quant ? (size_t)s.n_nodes * kQNodeWords * 4 : 0);
     void *buf = nullptr;
-    cudaError_t e = cudaMallocAsync(&buf, bytes, stream);
+    cudaError_t e = scratch_alloc(&buf, bytes, stream);
     if (e != cudaSuccess) return e;
     uint32_t *qnodes = quant ? (uint32_t *)((char *)buf + q_off) : nullptr;
     if (quant && s.n_nodes) {
@@ -550,7 +551,7 @@ cudaError_t launch_fwd_wave_3d(const SceneView<3> &s, const WalkParams &p, const
         wave_reduce_kernel<<<rblocks, kWalkBlock, 0, stream>>>(p, a, sum, sumsq, bounces, per_path);
         e = cudaGetLastError();
     }
-    const cudaError_t f = cudaFreeAsync(buf, stream);
+    const cudaError_t f = scratch_free(buf, stream);
     return e != cudaSuccess ? e : f;
 }
 

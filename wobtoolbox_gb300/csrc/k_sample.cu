@@ -13,6 +13,7 @@
 // prefix and the remaining rank, all on the caller's stream with no host round trip.
 #include "device_common.cuh"
 #include "launch.hpp"
+#include "scratch.hpp"
 
 #include <algorithm>
 
@@ -129,7 +130,7 @@ namespace wobgb {
 cudaError_t launch_clip_quantile(float *values, uint32_t n, float quantile, float *threshold, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
     void *scratch = nullptr;
-    cudaError_t e = cudaMallocAsync(&scratch, sizeof(ClipState) + 2048 * sizeof(uint32_t), stream);
+    cudaError_t e = scratch_alloc(&scratch, sizeof(ClipState) + 2048 * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     ClipState *st = (ClipState *)scratch;
     uint32_t *hist = (uint32_t *)((char *)scratch + sizeof(ClipState));
@@ -141,7 +142,7 @@ cudaError_t launch_clip_quantile(float *values, uint32_t n, float quantile, floa
     }
     clip_apply_kernel<<<(n + 255) / 256, 256, 0, stream>>>(values, n, st, threshold);
     e = cudaGetLastError();
-    const cudaError_t f = cudaFreeAsync(scratch, stream);
+    const cudaError_t f = scratch_free(scratch, stream);
     return e != cudaSuccess ? e : f;
 }
 

@@ -22,7 +22,8 @@ namespace {
 // the 2D double layer at >= 12 (1024-segment star: 2.87 ms against 3.88, 2.95 and 2.86 at >= 5, 8 and 10;
 // 8192 segments: 1.23 against 2.00, 1.45 and 1.33), the 3D forward walk on the wavefront (trace at >= 6 blocks/SM on
 // compressed nodes, 2^22-path chunks).
-std::atomic<int> g_config[kNumTunable] = {{1}, {3}, {1}, {3}};
+const int kDefaultConfig[kNumTunable] = {1, 3, 1, 3};
+std::atomic<int> g_config[kNumTunable] = {{-1}, {-1}, {-1}, {-1}};  // -1: the default
 const char *kFwdNames[kTuneOccupancies] = {"lockstep walk, >=5 blocks/SM", "wavefront, trace >=8 blocks/SM",
                                            "wavefront, trace >=6 blocks/SM",
                                            "wavefront, trace >=6 blocks/SM, 64-byte compressed nodes"};
@@ -43,7 +44,11 @@ int tunable_domain_variant(int dim, const WalkParams &p) {
     if (dim == 3 && st == kStratFwdSlNeumann) return 3;
     return -1;
 }
-int domain_config(int variant) { return (variant >= 0 && variant < kNumTunable) ? g_config[variant].load() : 0; }
+int domain_config(int variant) {
+    if (variant < 0 || variant >= kNumTunable) return 0;
+    const int c = g_config[variant].load();
+    return c >= 0 ? c : kDefaultConfig[variant];
+}
 void set_domain_config(int variant, int config) {
     if (variant >= 0 && variant < kNumTunable && config >= 0 && config < kTuneConfigs) g_config[variant].store(config);
 }
@@ -130,7 +135,18 @@ cudaError_t launch_domain_3d(const SceneView<3> &s, const WalkParams &p, const f
                              double *sum, double *sumsq, unsigned long long *bounces, float *per_path,
                              cudaStream_t stream) {
     const int v = tunable_domain_variant(3, p);
-    if (v >= 0) return launch_domain_config(3, v, domain_config(v), &s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
+    int config = domain_config(v);
+    if (v == 3 && g_config[3].load() < 0) {
+        // Unless a configuration was chosen: a forward walk whose warps are all resident in the lockstep
+        // kernel (5 blocks per SM, 97,280 paths) takes that; the wavefront's phases then have too few
+        // paths to fill (327,680 triangles, 4 bounces: 64,000 paths 0.85 ms lockstep, 1.07 wavefront;
+        // 128,000 paths 1.49 and 1.27).
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if ((uint64_t)n_points * ((p.n_paths + 31u) / 32u) <= (uint64_t)sms * 5u * (kWalkBlock / 32)) config = 0;
+    }
+    if (v >= 0) return launch_domain_config(3, v, config, &s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
     const int st = strategy_of(p.bie, p.estimator, p.problem);
     if (p.n_volume == 0 && st == kStratSingleLayer)
         return launch_domain_variant<3, kSingleLayer, kStratSingleLayer, false, 5>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);

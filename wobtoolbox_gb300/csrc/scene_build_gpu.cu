@@ -19,6 +19,7 @@
 
 #include "kahan_scan.hpp"
 #include "scene_host.hpp"
+#include "scratch.hpp"
 #include "sort_keys.hpp"
 
 #include <algorithm>
@@ -488,18 +489,18 @@ __global__ void k_offset_weights(uint32_t n, const float *__restrict__ delta, co
 // The build's scratch, one allocation: take() first adds up the sizes, after allocate() it hands out
 // the pointers in the same order.
 struct Tmp {
+    cudaStream_t stream;
     char *base = nullptr;
     size_t used = 0;
-    ~Tmp() {
-        if (base) cudaFree(base);
-    }
+    explicit Tmp(cudaStream_t st) : stream(st) {}
+    ~Tmp() { scratch_free(base, stream); }
     template <class T> void take(T **p, size_t count) {
         *p = base ? (T *)(base + used) : nullptr;
         used += (std::max<size_t>(count, 1) * sizeof(T) + 255) / 256 * 256;
     }
     cudaError_t allocate() {
         void *q = nullptr;
-        const cudaError_t e = cudaMalloc(&q, used);
+        const cudaError_t e = scratch_alloc(&q, used, stream);
         if (e == cudaSuccess) base = (char *)q;
         used = 0;
         return e;
@@ -511,7 +512,7 @@ inline uint32_t blocks(uint64_t n) { return (uint32_t)((n + kT - 1) / kT); }
 template <int D>
 std::string build_impl(uint32_t n, const float *verts, const float *normals, const float *bvals, const float *alphas,
                        const int32_t *types, cudaStream_t st, DeviceSceneBuild &out, cudaError_t &ce) {
-    Tmp tmp;
+    Tmp tmp(st);
 #define WOB_CK(x)                            \
     do {                                     \
         if ((ce = (x)) != cudaSuccess) return "CUDA error"; \

@@ -1,0 +1,67 @@
+// Scratch memory from a private stream-ordered pool per device. The default pool hands its memory back
+// to the driver at every synchronisation, and a call that follows one then maps it again: 0.85 ms for
+// the path state of a forward walk of 3.5 M paths (12.5 ms against 11.7 without a synchronisation
+// between calls), and some 0.2 ms for a device scene build's scratch (as cudaMalloc and cudaFree). The
+// pool is safe for any threads and streams; it is bounded (512 MB kept between calls) and trimmed when
+// the device's last scene goes.
+#include "scratch.hpp"
+
+#include <cstdint>
+#include <mutex>
+
+namespace wobgb {
+
+namespace {
+constexpr int kMaxDevices = 64;
+constexpr uint64_t kKeepBytes = 512ull << 20;
+std::mutex g_mutex;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+int g_scenes[kMaxDevices] = {};
+
+cudaError_t pool_of(int device, cudaMemPool_t *out) {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (!g_pool[device]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        uint64_t keep = kKeepBytes;
+        if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return e;
+        }
+        g_pool[device] = pool;
+    }
+    *out = g_pool[device];
+    return cudaSuccess;
+}
+}  // namespace
+
+cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    if (device < 0 || device >= kMaxDevices) return cudaMallocAsync(p, bytes, stream);
+    cudaMemPool_t pool;
+    if ((e = pool_of(device, &pool)) != cudaSuccess) return e;
+    return cudaMallocFromPoolAsync(p, bytes, pool, stream);
+}
+
+cudaError_t scratch_free(void *p, cudaStream_t stream) { return p ? cudaFreeAsync(p, stream) : cudaSuccess; }
+
+void scratch_retain(int device) {
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    g_scenes[device]++;
+}
+
+void scratch_release(int device) {
+    if (device < 0 || device >= kMaxDevices) return;
+    std::lock_guard<std::mutex> lock(g_mutex);
+    if (--g_scenes[device] == 0 && g_pool[device]) cudaMemPoolTrimTo(g_pool[device], 0);
+}
+
+}  // namespace wobgb
