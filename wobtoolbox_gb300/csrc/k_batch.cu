@@ -10,7 +10,7 @@
 
 namespace wobgb {
 
-constexpr int kBatchMinB = 8;  // 24 scenes: 12.6 ms at 5, 11.3 at 6, 11.1 at 8
+constexpr int kBatchMinB = 6;  // 24 scenes: 11.1 ms at 5, 10.5 at 6, 10.8 at 8
 
 // One unit (32 * ppt paths of one point) of a batched scene with the walker variant W; view and
 // p are the scene's view and parameters staged in shared memory by the warp.

@@ -360,15 +360,16 @@ template <int D, int kBie = -1, int kStrat = kStratRuntime, bool kVol = true, bo
     // Streaming RIS over K uniform candidates (scene.cuh:542-584, 847-889). A candidate's target
     // needs only its position, so the loop reads only the vertices of each candidate's element and
     // keeps the selected candidate's element (sel, 0xFFFFFFFF if none) and draws (su). The draws
-    // are taken in the reference's order -- candidate i's D draws, then its selection draw -- but
-    // candidate i + 1's draws and guide-table load are issued before candidate i's target is
-    // evaluated, so two dependent load chains are in flight instead of one.
+    // are taken in the reference's order -- candidate i's D draws, then its selection draw.
     //
-    // The loop is bound by issue and by the latency of its serial operations (3 "wait" stall cycles
-    // per instruction at 20 warps per SM). A candidate's D + 1 draws come from a window of two Philox
-    // blocks at one position, so a candidate costs one block at one call site instead of a refill
-    // check and a copy of the generator at each draw; the selection needs no division; and the
-    // target's quotients share reciprocals.
+    // The loop is bound by issue and by the latency of its serial operations, so candidates go kBatch at
+    // a time: their D + 1 draws each are a whole number of Philox blocks, cut out of a window of blocks
+    // at one position that stays the same from batch to batch (no refill checks, no branches), and
+    // their lookups, positions and targets are independent; only the running sum and the selection
+    // are serial. The selection needs no division, and the target's quotients share reciprocals. Against
+    // one candidate at a time: 100,000 paths x 1024 candidates 4.0 -> 3.7 ms, 64 right-hand sides 2.05 ->
+    // 2.00 ms, 24 batched scenes 10.7 -> 10.5 ms.
+    static constexpr int kBatch = D == 2 ? 4 : 2;
     __device__ __forceinline__ void ris_select(const BPoint<D> &yp, uint32_t &sel, float *su, float &w_sum,
                                                uint32_t &M) {
         sel = 0xFFFFFFFFu;
@@ -379,64 +380,73 @@ template <int D, int kBie = -1, int kStrat = kStratRuntime, bool kVol = true, bo
         const uint32_t K = p.n_resampling;
         if (K == 0) return;
         auto block = [&](uint32_t b) { return philox4x32_10(make_uint4(b, rng.c1, rng.c2, rng.c3), rng.k0, rng.k1); };
-        uint4 cur = rng.buf;         // the block holding the next draw, at position pos
-        uint32_t pos = (uint32_t)rng.used, next_block = rng.block;
-        if (pos == 4u) {
-            cur = block(next_block++);
-            pos = 0;
-        }
-        uint4 nxt = block(next_block++);
-        auto take = [&](float *u, float &r_sel) {
-            const bool odd = pos & 1u, high = pos & 2u;
-            auto pick = [&](uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-                const uint32_t x = high ? (odd ? d : c) : (odd ? b : a);
-                return (float)((x >> 8) + 1u) * 0x1p-24f;
-            };
-            u[0] = pick(cur.x, cur.y, cur.z, cur.w);
-            u[1] = pick(cur.y, cur.z, cur.w, nxt.x);
-            if constexpr (D == 2) {
-                r_sel = pick(cur.z, cur.w, nxt.x, nxt.y);
-                pos += 3u;
-            } else {
-                u[2] = pick(cur.z, cur.w, nxt.x, nxt.y);
-                r_sel = pick(cur.w, nxt.x, nxt.y, nxt.z);
-                pos += 4u;
-            }
-            if (pos >= 4u) {
-                pos -= 4u;
-                cur = nxt;
-                nxt = block(next_block++);
-            }
-        };
-        float u[D], r_sel;
-        take(u, r_sel);
-        uint4 g = __ldg(s.area_guide + guide_bin(s.area_G, u[0]));
-        for (uint32_t i = 0; i < K; i++) {
-            const uint32_t idx = cdf_resolve(s.area_cdf, g, u[0]);
-            const V<D> at = uniform_position<D>(s, idx, u);
-            float un[D], rn = 0.0f;
-#pragma unroll
-            for (int k = 0; k < D; k++) un[k] = 0.0f;
-            if (i + 1 < K) {
-                take(un, rn);
-                g = __ldg(s.area_guide + guide_bin(s.area_G, un[0]));
-            }
-            const float wi = ris_target_at(yp.type, yp, at) * s.total_area;
+        auto uniform_of = [](uint32_t x) { return (float)((x >> 8) + 1u) * 0x1p-24f; };
+        auto consider = [&](uint32_t idx, const float *u, float r_sel, float target) {
+            const float wi = target * s.total_area;
             w_sum = w_sum + wi;
             if (at_most_ratio(r_sel, wi, w_sum)) {
                 sel = idx;
 #pragma unroll
                 for (int k = 0; k < D; k++) su[k] = u[k];
             }
+        };
+        uint32_t i = 0;
+        if (K >= (uint32_t)kBatch) {
+            constexpr int kBlocks = kBatch * (D + 1) / 4;
+            static_assert(kBlocks * 4 == kBatch * (D + 1), "a batch's draws fill whole blocks");
+            uint4 W[kBlocks + 1];       // W[0]: the block of the next draw, at position pos
+            uint32_t pos = (uint32_t)rng.used, next_block = rng.block;
+            W[0] = rng.buf;
+            if (pos == 4u) {
+                W[0] = block(next_block++);
+                pos = 0;
+            }
+            const bool odd = pos & 1u, high = pos & 2u;
+            for (; i + kBatch <= K; i += kBatch) {
 #pragma unroll
-            for (int k = 0; k < D; k++) u[k] = un[k];
-            r_sel = rn;
+                for (int k = 1; k <= kBlocks; k++) W[k] = block(next_block++);
+                auto word = [&](int w) {
+                    const uint4 &v = W[w >> 2];
+                    return (w & 3) == 0 ? v.x : (w & 3) == 1 ? v.y : (w & 3) == 2 ? v.z : v.w;
+                };
+                auto draw = [&](int d) {  // draw d of the batch: word pos + d
+                    return uniform_of(high ? (odd ? word(d + 3) : word(d + 2)) : (odd ? word(d + 1) : word(d)));
+                };
+                float u[kBatch][D], r_sel[kBatch], target[kBatch];
+                uint32_t idx[kBatch];
+                uint4 g[kBatch];
+#pragma unroll
+                for (int c = 0; c < kBatch; c++) {
+#pragma unroll
+                    for (int k = 0; k < D; k++) u[c][k] = draw(c * (D + 1) + k);
+                    r_sel[c] = draw(c * (D + 1) + D);
+                    g[c] = __ldg(s.area_guide + guide_bin(s.area_G, u[c][0]));
+                }
+#pragma unroll
+                for (int c = 0; c < kBatch; c++) idx[c] = cdf_resolve(s.area_cdf, g[c], u[c][0]);
+                V<D> at[kBatch];
+#pragma unroll
+                for (int c = 0; c < kBatch; c++) at[c] = uniform_position<D>(s, idx[c], u[c]);
+#pragma unroll
+                for (int c = 0; c < kBatch; c++) target[c] = ris_target_at(yp.type, yp, at[c]);
+#pragma unroll
+                for (int c = 0; c < kBatch; c++) consider(idx[c], u[c], r_sel[c], target[c]);
+                W[0] = W[kBlocks];
+            }
+            // the stream as single draws leave it: W[0] is loaded, pos of its words are used
+            rng.buf = W[0];
+            rng.used = (int)pos;
+            rng.block = next_block;
+        }
+        for (; i < K; i++) {
+            float u[D];
+#pragma unroll
+            for (int k = 0; k < D; k++) u[k] = rng.uniform();
+            const float r_sel = rng.uniform();
+            const uint32_t idx = cdf_search(s.area_cdf, s.area_guide, s.area_G, u[0]);
+            consider(idx, u, r_sel, ris_target_at(yp.type, yp, uniform_position<D>(s, idx, u)));
         }
         M = K;
-        // the stream as K (D + 1) single draws leave it: cur is loaded, pos of its words are used
-        rng.buf = cur;
-        rng.used = (int)pos;
-        rng.block = next_block - 1u;
     }
     __device__ __forceinline__ BPoint<D> sample_ris(const BPoint<D> &yp, float &inv_pdf) {
         uint32_t sel, M;
