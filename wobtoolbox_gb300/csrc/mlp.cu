@@ -427,7 +427,7 @@ struct wob_mlp_s {
         cudaError_t e = ensure(batch);
         if (e != cudaSuccess) return e;
         if (!sched && (e = cudaMalloc(&sched, 16)) != cudaSuccess) return e;
-        if (!step && (e = cudaMalloc(&step, 8)) != cudaSuccess) return e;
+        if (!step && (e = cudaMalloc(&step, 12)) != cudaSuccess) return e;
         if (batch <= train_cap) return cudaSuccess;
         for (float **p : {&xb, &tb}) {
             if (*p) cudaFree(*p);
@@ -443,7 +443,7 @@ struct wob_mlp_s {
     bool fused_ok() const { return hidden == 4 && n_freq == 32 && out_dim <= 64; }
     cudaError_t ensure_fused(uint32_t batch) {
         cudaError_t e;
-        if (!step && (e = cudaMalloc(&step, 8)) != cudaSuccess) return e;
+        if (!step && (e = cudaMalloc(&step, 12)) != cudaSuccess) return e;
         if (!image) {
             const size_t bytes = wobgb::fused_train_image_words() * 4;
             if ((e = cudaMalloc(&image, bytes)) != cudaSuccess || (e = cudaMemset(image, 0, bytes)) != cudaSuccess)
@@ -458,7 +458,7 @@ struct wob_mlp_s {
             if (*p) cudaFree(*p);
             *p = nullptr;
         }
-        if ((e = cudaMalloc(&partial, (size_t)blocks * n_params * 4)) != cudaSuccess ||
+        if ((e = cudaMalloc(&partial, (size_t)blocks * wobgb::fused_train_partial_words(out_dim) * 4)) != cudaSuccess ||
             (e = cudaMalloc(&partial_loss, (size_t)blocks * 4)) != cudaSuccess)
             return e;
         partial_blocks = blocks;
@@ -700,7 +700,7 @@ int wob_mlp_gradient_fused(wob_mlp m, const float *inputs, const float *targets,
     cudaError_t e = m->ensure_fused(n);
     if (e != cudaSuccess) return mfail_cuda(e, "MLP training workspace");
     if ((e = cudaMemsetAsync(m->step, 0, 8, st)) != cudaSuccess) return mfail_cuda(e, "MLP step counter");
-    wobgb::FusedTrainArgs a{m->params, m->freqs, inputs, targets, n, m->out_dim, n, m->n_params, 0u, 0ull, m->step,
+    wobgb::FusedTrainArgs a{m->params, m->freqs, inputs, targets, n, m->out_dim, n, m->n_params, 0u, 0u, 0ull, m->step,
                             m->partial, m->partial_loss, m->image, m->err, m->inject_wait_polls};
     e = wobgb::launch_fused_gradient(a, grad, loss, st);
     return e == cudaSuccess ? WOB_OK : mfail_cuda(e, "fused MLP gradient");
@@ -750,9 +750,9 @@ int wob_mlp_train(wob_mlp m, const float *inputs, const float *targets, uint32_t
         cleanup();
         return mfail_cuda(e, "capturing the training step");
     }
-    auto one_step = [&]() -> cudaError_t {
+    auto one_step = [&](uint32_t early) -> cudaError_t {
         if (fused) {
-            FusedTrainArgs a{m->params, m->freqs, inputs, targets, n, m->out_dim, batch, m->n_params, 1u, seed, m->step,
+            FusedTrainArgs a{m->params, m->freqs, inputs, targets, n, m->out_dim, batch, m->n_params, 1u, early, seed, m->step,
                              m->partial, m->partial_loss, m->image, m->err, m->inject_wait_polls};
             return launch_fused_train_step(a, m->params, m->adam_m, m->adam_v, steps, lr, adam_base, loss_history, cs);
         }
@@ -766,7 +766,7 @@ int wob_mlp_train(wob_mlp m, const float *inputs, const float *targets, uint32_t
         return eb != cudaSuccess ? eb : cudaGetLastError();
     };
     cudaError_t e_body = cudaSuccess;
-    for (uint32_t i = 0; i < kSteps && e_body == cudaSuccess; i++) e_body = one_step();
+    for (uint32_t i = 0; i < kSteps && e_body == cudaSuccess; i++) e_body = one_step(i > 0);
     e = cudaStreamEndCapture(cs, &graph);
     if (e_body != cudaSuccess || e != cudaSuccess || (e = cudaGraphInstantiate(&exec, graph, 0)) != cudaSuccess) {
         cleanup();
@@ -778,7 +778,7 @@ int wob_mlp_train(wob_mlp m, const float *inputs, const float *targets, uint32_t
             return mfail_cuda(e, "launching the training steps");
         }
     for (uint32_t i = 0; i < steps % kSteps; i++)
-        if ((e = one_step()) != cudaSuccess) {
+        if ((e = one_step(i > 0)) != cudaSuccess) {
             cleanup();
             return mfail_cuda(e, "launching a training step");
         }
