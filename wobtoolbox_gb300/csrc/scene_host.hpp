@@ -105,8 +105,8 @@ std::string build_host_scene(int dim, uint32_t n, const float *verts, const floa
 // most 2^22 (key G then keeps its rounding under a quarter bin). With one record per entry a lookup
 // spans two bins and on average two boundaries, and in most warps some lane falls through the
 // record's two CDF values into the bisection's dependent loads; with four per entry that is rare: the
-// Robin walk on 81,920 triangles went from 25.7 to 24.4 ms (37.5 to 29.4 without a register cap), 64-candidate resampling for 64 right-hand sides from
-// 2.43 to 2.06 ms. Above 2^20 records the table would crowd the element records out of the L2.
+// Robin walk on 81,920 triangles went from 25.7 to 24.4 ms (37.5 to 29.4 without a register cap),
+// 64-candidate resampling for 64 right-hand sides from 2.43 to 2.06 ms. Above 2^20 records the table would crowd the element records out of the L2.
 inline uint32_t guide_records(uint32_t n) {
     const uint64_t four = 4 * (uint64_t)n, wide = four < (1u << 20) ? four : (1u << 20);
     const uint64_t g = wide > n ? wide : n;
