@@ -369,7 +369,7 @@ uint32_t chunk_length(uint32_t n) {
 // Guide tables: a block's kGuideBlock records need the first indices of kGuideBlock + 2 thresholds. Two
 // warps find the first and the last of them by a 32-way search (four dependent loads for a million
 // elements instead of twenty), the CDF between them is staged in shared memory, and every thread
-// searches there: a full search per record took 43 us for 327,680 records, this 14 us for 1,048,576.
+// searches there (a full search per record took 43 us for 327,680 records, about ten times this).
 constexpr int kGuideBlock = 256;
 constexpr uint32_t kGuideStage = 2048;
 // The least float not below the host's threshold, the double nearest (j - 1/2) / G: a float is below one
