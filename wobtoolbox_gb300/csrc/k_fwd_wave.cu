@@ -264,7 +264,12 @@ __device__ __forceinline__ uint32_t qnode_hits(const uint32_t *__restrict__ qn, 
 // visit, the test of one held leaf, or the choice of the hit and the fetch of the next query.
 // Descending in every lane until its leaves were held, then testing them all, kept 11.5 of 32 lanes
 // active (ALU pipe 66 %: issue-bound), because both loops run as long as their longest lane. Leaves
-// queue in the order they are met, so the hits keep their order.
+// queue in the order they are met, so the hits keep their order. A finished lane counts kDoneVotes
+// times: it idles until its step is taken, where a lane that waits with a node and a leaf may have
+// the other one run. On 327,680 triangles, 54,025 points x 64 paths, by resident blocks per SM and votes:
+//   6: 11.75 ms (1), 11.4 (2)   8: 11.0 (1), 10.7 (2), 10.7 (3), 10.9 (4)   9: 11.0 (1), 10.5 (2), 10.7 (3)
+//   7: 12.2 (1)   10: 11.4 (1)   at 6, a node counting twice 12.0, a leaf twice 12.8.
+constexpr int kDoneVotes = 2;
 template <int kMinB, int kLeaves, bool kQuant>
 __global__ void __launch_bounds__(kWalkBlock, kMinB) wave_trace_kernel(SceneView<3> s, WalkParams p, WaveArgs a,
                                                                       const uint32_t *__restrict__ qnodes) {
@@ -308,7 +313,7 @@ __global__ void __launch_bounds__(kWalkBlock, kMinB) wave_trace_kernel(SceneView
         const uint32_t need = __ballot_sync(kFull, fetch || done);
         const int n_done = __popc(need);
         if (n_node == 0 && n_leaf == 0 && n_done == 0) break;
-        if (n_node >= n_leaf && n_node >= n_done) {
+        if (n_node >= n_leaf && n_node >= kDoneVotes * n_done) {
             if (node) {
                 if (++steps > s.traversal_limit) {
                     atomicOr(s.err, kErrTraversalLimit);
@@ -358,7 +363,7 @@ __global__ void __launch_bounds__(kWalkBlock, kMinB) wave_trace_kernel(SceneView
                     advance();
                 }
             }
-        } else if (n_leaf >= n_done) {
+        } else if (n_leaf >= kDoneVotes * n_done) {
             if (held) {
                 const uint32_t leaf = my_leaf[(head & (kLeaves - 1u)) * kWalkBlock];
                 head++;
@@ -540,7 +545,7 @@ cudaError_t launch_fwd_wave_3d(const SceneView<3> &s, const WalkParams &p, const
             switch (shape) {
             case 1: e = trace<8, 8, false>(s, p, a, nullptr, stream); break;
             case 2: e = trace<6, 8, false>(s, p, a, nullptr, stream); break;
-            default: e = trace<6, 8, true>(s, p, a, qnodes, stream); break;
+            default: e = trace<9, 8, true>(s, p, a, qnodes, stream); break;
             }
             if (e != cudaSuccess) break;
             wave_consume_kernel<<<blocks, kWalkBlock, 0, stream>>>(s, p, a, m);

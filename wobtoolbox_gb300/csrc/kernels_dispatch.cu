@@ -20,13 +20,13 @@ namespace {
 // (81,920-triangle Robin slice, 512 paths: 24.4 ms against 25.0 at >= 5, 36.0 at >= 10 and, before, 37.8
 // without a register cap; direct Neumann on 81,920 triangles: 3.97 ms against 4.39, 4.01 and 4.52),
 // the 2D double layer at >= 12 (1024-segment star: 2.87 ms against 3.88, 2.95 and 2.86 at >= 5, 8 and 10;
-// 8192 segments: 1.23 against 2.00, 1.45 and 1.33), the 3D forward walk on the wavefront (trace at >= 6 blocks/SM on
+// 8192 segments: 1.23 against 2.00, 1.45 and 1.33), the 3D forward walk on the wavefront (trace at >= 9 blocks/SM on
 // compressed nodes, 2^22-path chunks).
 const int kDefaultConfig[kNumTunable] = {1, 3, 1, 3};
 std::atomic<int> g_config[kNumTunable] = {{-1}, {-1}, {-1}, {-1}};  // -1: the default
 const char *kFwdNames[kTuneOccupancies] = {"lockstep walk, >=5 blocks/SM", "wavefront, trace >=8 blocks/SM",
                                            "wavefront, trace >=6 blocks/SM",
-                                           "wavefront, trace >=6 blocks/SM, 64-byte compressed nodes"};
+                                           "wavefront, trace >=9 blocks/SM, 64-byte compressed nodes"};
 const uint32_t kWaveSlotsOf[kTunePptCaps] = {1u << 22, 1u << 21, 1u << 20, 1u << 19};
 const int kMinBOf[kTuneOccupancies] = {5, 8, 10, 12};
 const uint32_t kPptCapOf[kTunePptCaps] = {0u, 4u, 2u, 1u};
