@@ -54,6 +54,10 @@ cudaError_t scratch_free(void *p, cudaStream_t stream) { return p ? cudaFreeAsyn
 
 void scratch_retain(int device) {
     if (device < 0 || device >= kMaxDevices) return;
+    // the pool exists before any walk, so that none makes it on a capturing stream (a failure here is
+    // reported by the first allocation, which tries again)
+    cudaMemPool_t pool;
+    if (pool_of(device, &pool) != cudaSuccess) cudaGetLastError();
     std::lock_guard<std::mutex> lock(g_mutex);
     g_scenes[device]++;
 }

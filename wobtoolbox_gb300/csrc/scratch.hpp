@@ -11,8 +11,8 @@ namespace wobgb {
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream);
 cudaError_t scratch_free(void *p, cudaStream_t stream);
 
-// A scene on `device` begins / ends its life. The pool keeps up to 512 MB between calls while a scene
-// of the device lives; the last one to go gives it back.
+// A scene on `device` begins / ends its life. The first makes the pool, which keeps up to 512 MB between
+// calls while a scene of the device lives; the last one to go gives it back.
 void scratch_retain(int device);
 void scratch_release(int device);
 
