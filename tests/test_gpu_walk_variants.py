@@ -139,6 +139,28 @@ def test_packed_vpl_sums(engine, oracle, cuda, n_vpl):
     scene.close()
 
 
+@pytest.mark.parametrize("eps", [1e-30, float("inf")])
+@pytest.mark.parametrize("n_vpl", [130, 2100, 4100])
+def test_packed_vpl_sums_infinite(engine, oracle, cuda, n_vpl, eps):
+    """Infinite logarithms (a point on a VPL with eps^2 = 0, eps = inf) of one sign, the second tile of a
+    pair shorter than the first or missing: infinities stay infinities."""
+    torch = cuda
+    verts, nrm, data, ty, _ = W.vpl_flow_scene()
+    scene = engine.SceneHost(verts, nrm, data, ty)
+    rng = np.random.default_rng(n_vpl)
+    vp = rng.uniform(-0.5, 0.5, (n_vpl, 2)).astype(F32)
+    mu = rng.uniform(0.5, 1.0, n_vpl).astype(F32)
+    pts = vp[[0, 51, 100, n_vpl - 1]].copy()
+    s = torch.zeros(len(pts), 3, dtype=torch.float64, device="cuda")
+    scene.vpl_aggregate(eps, torch.from_numpy(vp).cuda(), torch.from_numpy(mu).cuda(), n_vpl,
+                        torch.from_numpy(pts).cuda(), len(pts), s)
+    torch.cuda.synchronize()
+    want = oracle.vpl_aggregate(2, scene.info()["total_area"], eps, vp, mu, pts)
+    assert np.isinf(want[:, 0]).all()
+    assert np.array_equal(s.cpu().numpy(), want, equal_nan=True)
+    scene.close()
+
+
 @pytest.mark.parametrize("n,hidden,out_dim", [(1, 4, 1), (15, 1, 3), (16, 4, 64), (17, 16, 1), (129, 4, 9), (5000, 2, 8)])
 def test_inference_is_the_layerwise_network(engine, cuda, n, hidden, out_dim):
     """The gradient's layer-by-layer forward pass against the one-kernel inference: with its outputs as

@@ -163,8 +163,10 @@ __global__ void __launch_bounds__(32 * kVplSplit, 4) vpl_aggregate2_kernel(const
                     auto weight = [&](float kw, float v) {
                         return v >= eps2 ? kw / v : (v > 0.0f ? kw / (sqrtf(v) * eps) : 0.0f);
                     };
-                    u = f2(k.x * log_own(fmax_ref(qa, eps2)), k.y * log_own(fmax_ref(qb, eps2)));
-                    g = f2(weight(k.z, qa), weight(k.w, qb));
+                    // beyond a shorter second tile its half adds zero, also where the logarithm is infinite
+                    const bool second = h + j < mb;
+                    u = f2(k.x * log_own(fmax_ref(qa, eps2)), second ? k.y * log_own(fmax_ref(qb, eps2)) : 0.0f);
+                    g = f2(weight(k.z, qa), second ? weight(k.w, qb) : 0.0f);
                 }
                 part[0] = f2add(part[0], u);
                 part[1] = f2add(part[1], f2mul(g, r0, z));
