@@ -161,6 +161,26 @@ def test_packed_vpl_sums_infinite(engine, oracle, cuda, n_vpl, eps):
     scene.close()
 
 
+@pytest.mark.parametrize("at", [5, 2055])
+def test_packed_vpl_sums_nan(engine, oracle, cuda, at):
+    """A VPL without a coordinate in one half of a pair only: as in the scalar sums, not a finite value."""
+    torch = cuda
+    verts, nrm, data, ty, _ = W.vpl_flow_scene()
+    scene = engine.SceneHost(verts, nrm, data, ty)
+    rng = np.random.default_rng(at)
+    vp = rng.uniform(-0.5, 0.5, (2100, 2)).astype(F32)
+    vp[at, 0] = np.nan
+    mu = rng.uniform(0.5, 1.0, len(vp)).astype(F32)
+    pts = rng.uniform(-0.5, 0.5, (5, 2)).astype(F32)
+    s = torch.zeros(len(pts), 3, dtype=torch.float64, device="cuda")
+    scene.vpl_aggregate(1e-4, torch.from_numpy(vp).cuda(), torch.from_numpy(mu).cuda(), len(vp),
+                        torch.from_numpy(pts).cuda(), len(pts), s)
+    torch.cuda.synchronize()
+    want = oracle.vpl_aggregate(2, scene.info()["total_area"], 1e-4, vp, mu, pts)
+    assert np.array_equal(s.cpu().numpy(), want, equal_nan=True)
+    scene.close()
+
+
 @pytest.mark.parametrize("n,hidden,out_dim", [(1, 4, 1), (15, 1, 3), (16, 4, 64), (17, 16, 1), (129, 4, 9), (5000, 2, 8)])
 def test_inference_is_the_layerwise_network(engine, cuda, n, hidden, out_dim):
     """The gradient's layer-by-layer forward pass against the one-kernel inference: with its outputs as

@@ -109,6 +109,13 @@ __global__ void __launch_bounds__(32 * kVplSplit) vpl_aggregate3_kernel(const fl
 // range (q below eps^2 or beyond 2^60, or a weight out of the quotient's range) take the scalar
 // expressions. The kernel above is bound by issue, 85 instructions a pair; a packed one is issued for
 // two pairs: 100,000 VPLs x 39,280 points 10.2 -> 5.7 ms.
+// The smaller of two floats, NaN if either is (fminf returns the other one).
+__device__ __forceinline__ float fmin_nan(float a, float b) {
+    float m;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+
 constexpr int kStage = 128;  // VPLs of each tile staged in shared memory at a time
 
 __global__ void __launch_bounds__(32 * kVplSplit, 4) vpl_aggregate2_kernel(const float *__restrict__ vpl_p,
@@ -156,7 +163,7 @@ __global__ void __launch_bounds__(32 * kVplSplit, 4) vpl_aggregate2_kernel(const
                 const F2 q = f2add(f2mul(r0, r0, z), f2mul(r1, r1, z));
                 const float qa = f2lo(q), qb = f2hi(q);
                 F2 u, g;
-                if (__builtin_expect(!plain && fminf(qa, qb) >= lo && fmaxf(qa, qb) <= 0x1p60f, 1)) {
+                if (__builtin_expect(!plain && fmin_nan(qa, qb) >= lo && fmaxf(qa, qb) <= 0x1p60f, 1)) {
                     u = f2mul(f2(k.x, k.y), f2log(q, z), z);
                     g = f2quotient(f2(k.z, k.w), q, z);
                 } else {
