@@ -322,14 +322,14 @@ int wob_device_info(int *device, int *sm_count) {
     return WOB_OK;
 }
 
-// The 2D segments' endpoints packed from the element records.
-static cudaError_t pack_segments(wob_scene_s *s) {
-    if (s->host.line_grid.K == 0) return cudaSuccess;
-    const size_t bytes = (size_t)s->host.n * 16;
-    cudaError_t e = cudaMalloc(&s->lg_seg.ptr, bytes);
-    if (e != cudaSuccess) return e;
-    s->lg_seg.bytes = bytes;
-    return cudaMemcpy2D(s->lg_seg.ptr, 16, s->elems.ptr, 64, 16, s->host.n, cudaMemcpyDeviceToDevice);
+// The 2D segments' endpoints packed from the element records (scenes with a line grid).
+static std::vector<float> packed_segments(const wobgb::HostScene &h) {
+    std::vector<float> seg;
+    if (h.line_grid.K == 0) return seg;
+    const size_t stride = (size_t)wobgb::elem_record_floats(h.dim);
+    seg.reserve((size_t)h.n * 4);
+    for (size_t i = 0; i < h.n; i++) seg.insert(seg.end(), h.elems.begin() + i * stride, h.elems.begin() + i * stride + 4);
+    return seg;
 }
 
 static int scene_create_impl(int dim, uint32_t n_elems, const float *vertices, const float *normals,
@@ -353,6 +353,7 @@ static int scene_create_impl(int dim, uint32_t n_elems, const float *vertices, c
     const wobgb::HostScene &h = s->host;
     s->area_G = (uint32_t)(h.area_guide.size() / 4);
     s->bv_G = (uint32_t)(h.bv_guide.size() / 4);
+    const std::vector<float> seg = packed_segments(h);
     const uint32_t zero = 0;
     if ((e = upload(s->elems, h.elems.data(), h.elems.size() * 4)) != cudaSuccess ||
         (e = upload(s->elem_aux, h.elem_aux.data(), h.elem_aux.size() * 4)) != cudaSuccess ||
@@ -362,11 +363,14 @@ static int scene_create_impl(int dim, uint32_t n_elems, const float *vertices, c
         (e = upload(s->area_guide, h.area_guide.data(), h.area_guide.size() * 4)) != cudaSuccess ||
         (e = upload(s->bv_cdf, h.bv_cdf.data(), h.bv_cdf.size() * 4)) != cudaSuccess ||
         (e = upload(s->bv_guide, h.bv_guide.data(), h.bv_guide.size() * 4)) != cudaSuccess ||
-        (e = upload(s->err, &zero, 4)) != cudaSuccess ||
         (e = upload(s->lg_bins, h.line_grid.bins.data(), h.line_grid.bins.size() * 4)) != cudaSuccess ||
         (e = upload(s->lg_off, h.line_grid.offsets.data(), h.line_grid.offsets.size() * 4)) != cudaSuccess ||
         (e = upload(s->lg_ent, h.line_grid.entries.data(), h.line_grid.entries.size() * 2)) != cudaSuccess ||
-        (e = pack_segments(s)) != cudaSuccess) {
+        (e = upload(s->lg_seg, seg.data(), seg.size() * 4)) != cudaSuccess ||
+        (e = upload(s->err, &zero, 4)) != cudaSuccess ||
+        // a copy from pageable memory may return before its last bytes have landed, and a walk on a
+        // non-blocking stream is not ordered after the legacy stream's copies
+        (e = cudaStreamSynchronize(nullptr)) != cudaSuccess) {
         s->release_all();
         return fail_cuda(e, "uploading the scene");
     }
