@@ -114,7 +114,7 @@ __device__ __forceinline__ float closest_value(const SceneView<2> &s, const Clos
 // of three states -- a node to visit, a leaf to test, a finished query -- and the warp executes, each
 // iteration, the step most of its lanes wait for (finished queries count half: 5.0 ms against 5.4 with
 // equal weights). A query starts from the distance to the previous
-// jump's closest element, which prunes its first descent, and keeps box distances on the stack, so
+// jump's closest element (where that is finite), which prunes its first descent, and keeps box distances on the stack, so
 // that children the best distance has passed are dropped unvisited; children are ordered by a
 // register network. All paths of a point share the first query. The closest element, the
 // lexicographic minimum of (distance, index) over all elements, does not depend on any of this.
@@ -286,6 +286,12 @@ __global__ void __launch_bounds__(kBlock, 8) wos_kernel(SceneView<2> s, WalkPara
                     sp = 0;
                     steps = 1;
                     waiting = false;
+                    if (__builtin_expect(!(c.d2 < INFINITY), 0)) {
+                        // a walk outside that has left the float range: the query starts from nothing, and
+                        // a position that is not a number has no closest element
+                        waiting = !(x.v[0] == x.v[0] && x.v[1] == x.v[1]);
+                        c = Closest{INFINITY, 0xFFFFFFFFu, 0.0f};
+                    }
                 }
             }
         }
