@@ -635,6 +635,7 @@ int wob_mlp_set_params(wob_mlp m, const float *params) {
 int wob_mlp_forward(wob_mlp m, const float *inputs, uint32_t n, float *outputs, void *stream) {
     if (!m || (!inputs && n) || (!outputs && n)) return mfail(WOB_ERR_INVALID_ARGUMENT, "mlp, inputs and outputs are required");
     if (n == 0) return WOB_OK;
+    std::lock_guard<std::mutex> lock(m->mu);  // waits for a training call, which rewrites the parameters
     using namespace wobgb;
     const InferArgs a{m->params, m->freqs, inputs, outputs, n, m->hidden, m->out_dim};
     const size_t smem = infer_smem(m->hidden);
