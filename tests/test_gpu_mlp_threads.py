@@ -53,3 +53,43 @@ def test_inference_beside_training_sees_whole_steps(engine, cuda):
     for k, y in seen:
         assert np.array_equal(y, whole[k]) or np.array_equal(y, whole[k + 1])
     mlp.close()
+
+
+def test_inference_of_networks_of_different_depth(engine, cuda):
+    """Networks of different depths, which need different amounts of shared memory, evaluated from two
+    threads at once: every call is accepted and gives what it gives alone."""
+    from wobtoolbox_gb300 import cv
+    torch = cuda
+    n = 64
+    x = torch.randn(n, 6, generator=torch.Generator().manual_seed(1)).cuda()
+    nets = [cv.MLP(32, hidden, 1, 1.0, hidden) for hidden in (16, 8)]
+    outs = [torch.zeros(n, 1, device="cuda") for _ in nets]
+    streams = [torch.cuda.Stream() for _ in nets]
+    alone = []
+    torch.cuda.synchronize()
+    for net, out, st in zip(nets, outs, streams):
+        net.forward(x, n, out, st)
+        st.synchronize()
+        alone.append(out.clone())
+        out.zero_()
+    torch.cuda.synchronize()
+    failed = []
+
+    def loop(i):
+        torch.cuda.set_device(0)
+        try:
+            for _ in range(5000):
+                nets[i].forward(x, n, outs[i], streams[i])
+        except Exception as ex:  # noqa: BLE001 - reported by the assertion below
+            failed.append(repr(ex))
+
+    threads = [threading.Thread(target=loop, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed, failed
+    for net, out, want in zip(nets, outs, alone):
+        assert torch.equal(out, want)
+        net.close()

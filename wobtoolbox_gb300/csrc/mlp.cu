@@ -173,6 +173,7 @@ __global__ void fourier_kernel(const float *__restrict__ in, const float *__rest
 // row); mma.sync rather than tcgen05 because the products are a twentieth of that issue.
 // ------------------------------------------------------------------------------------------
 constexpr int kInferWarps = 8;
+constexpr uint32_t kMaxHidden = 16;  // wob_mlp_create
 constexpr int kWPad = kWidth + 8;  // BF16 values per weight row in shared memory
 
 struct InferArgs {
@@ -557,7 +558,7 @@ int wob_mlp_create(uint32_t n_freq, uint32_t hidden_layers, uint32_t out_dim, fl
     if (!out) return mfail(WOB_ERR_INVALID_ARGUMENT, "out is NULL");
     *out = nullptr;
     if (2 * n_freq != (uint32_t)wobgb::kWidth) return mfail(WOB_ERR_UNSUPPORTED, "2 * n_freq must equal the width 64");
-    if (hidden_layers < 1 || hidden_layers > 16) return mfail(WOB_ERR_INVALID_ARGUMENT, "hidden_layers must be 1..16");
+    if (hidden_layers < 1 || hidden_layers > wobgb::kMaxHidden) return mfail(WOB_ERR_INVALID_ARGUMENT, "hidden_layers must be 1..16");
     if (out_dim < 1 || out_dim > 64) return mfail(WOB_ERR_INVALID_ARGUMENT, "out_dim must be 1..64");
     if (!(freq_sigma > 0.0f)) return mfail(WOB_ERR_INVALID_ARGUMENT, "freq_sigma must be positive");
     wob_mlp_s *m = new wob_mlp_s();
@@ -640,8 +641,11 @@ int wob_mlp_forward(wob_mlp m, const float *inputs, uint32_t n, float *outputs, 
     const InferArgs a{m->params, m->freqs, inputs, outputs, n, m->hidden, m->out_dim};
     const size_t smem = infer_smem(m->hidden);
     cudaError_t e = cudaSuccess;
+    // the limit belongs to the kernel, which networks of other depths launch from other threads: always
+    // the deepest network's
     if (smem > 48u * 1024u &&
-        (e = cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        (e = cudaFuncSetAttribute(infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)infer_smem(kMaxHidden))) != cudaSuccess)
         return mfail_cuda(e, "MLP forward");
     int dev = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
