@@ -430,15 +430,15 @@ __global__ void __launch_bounds__(kCvBlock, 4) cv_sum_kernel(SceneView<3> s, con
             a[3] += sg * G[2];
         }
     };
-    // a source by the centroid rule (0 where `near`)
+    // a source by the centroid rule (0 where `near`, also for a density that is not finite)
     auto centroid_rule = [&](const float4 &q, float dx, float dy, float dz, float r2, bool near) {
-        const float rinv = near ? 0.0f : rsqrtf(r2);
+        const float rinv = near ? 0.0f : rsqrtf(r2), w = near ? 0.0f : q.w;
         const float r3 = rinv * rinv * rinv;
         if (kMode == 0) {
-            a[0] += q.w * (dx * nn[0] + dy * nn[1] + dz * nn[2]) * r3;
+            a[0] += w * (dx * nn[0] + dy * nn[1] + dz * nn[2]) * r3;
         } else {
-            a[0] += q.w * rinv;
-            const float wr3 = q.w * r3;
+            a[0] += w * rinv;
+            const float wr3 = w * r3;
             a[1] -= wr3 * dx;
             a[2] -= wr3 * dy;
             a[3] -= wr3 * dz;
