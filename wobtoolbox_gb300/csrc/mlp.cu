@@ -15,6 +15,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -638,9 +639,17 @@ int wob_mlp_forward(wob_mlp m, const float *inputs, uint32_t n, float *outputs, 
     if (n == 0) return WOB_OK;
     std::lock_guard<std::mutex> lock(m->mu);  // waits for a training call, which rewrites the parameters
     using namespace wobgb;
+    cudaError_t e = cudaSuccess;
+    const size_t n_in = (size_t)n * kFeatIn, n_out = (size_t)n * m->out_dim;
+    if ((uintptr_t)inputs < (uintptr_t)(outputs + n_out) && (uintptr_t)outputs < (uintptr_t)(inputs + n_in)) {
+        // outputs over the inputs: layer by layer, which has read every input before the first output is written
+        if ((e = m->ensure(n)) != cudaSuccess) return mfail_cuda(e, "MLP workspace");
+        if ((e = forward_impl(m, inputs, n, (cudaStream_t)stream)) != cudaSuccess) return mfail_cuda(e, "MLP forward");
+        e = cudaMemcpyAsync(outputs, m->Y, n_out * 4, cudaMemcpyDeviceToDevice, (cudaStream_t)stream);
+        return e == cudaSuccess ? WOB_OK : mfail_cuda(e, "MLP forward copy");
+    }
     const InferArgs a{m->params, m->freqs, inputs, outputs, n, m->hidden, m->out_dim};
     const size_t smem = infer_smem(m->hidden);
-    cudaError_t e = cudaSuccess;
     // the limit belongs to the kernel, which networks of other depths launch from other threads: always
     // the deepest network's
     if (smem > 48u * 1024u &&
