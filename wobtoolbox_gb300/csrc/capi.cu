@@ -400,6 +400,7 @@ static int scene_create_device_impl(int dim, uint32_t n_elems, const float *vert
     if (e != cudaSuccess) {
         return fail_cuda(e, "cudaGetDevice");
     }
+    s->count();  // the build's own scratch comes from the pool
     wobgb::DeviceSceneBuild b;
     std::string err = wobgb::build_device_scene(dim, n_elems, vertices, normals, boundary_values, robin_alphas,
                                                 boundary_types, (cudaStream_t)stream, b, e);
@@ -435,7 +436,6 @@ static int scene_create_device_impl(int dim, uint32_t n_elems, const float *vert
         s->release_all();
         return fail_cuda(e, "allocating the error word");
     }
-    s->count();
     *out = owner.release();
     return WOB_OK;
 }

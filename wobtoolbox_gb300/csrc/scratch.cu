@@ -18,47 +18,44 @@ std::mutex g_mutex;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 int g_scenes[kMaxDevices] = {};
 
-cudaError_t pool_of(int device, cudaMemPool_t *out) {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    if (!g_pool[device]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t pool = nullptr;
-        cudaError_t e = cudaMemPoolCreate(&pool, &props);
-        if (e != cudaSuccess) return e;
-        uint64_t keep = kKeepBytes;
-        if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
-            cudaMemPoolDestroy(pool);
-            return e;
-        }
-        g_pool[device] = pool;
+cudaError_t make_pool(int device) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = cudaMemPoolCreate(&pool, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = kKeepBytes;
+    if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+        cudaMemPoolDestroy(pool);
+        return e;
     }
-    *out = g_pool[device];
+    g_pool[device] = pool;
     return cudaSuccess;
 }
 }  // namespace
 
+// A pool cannot be made while a stream is being captured, so no allocation makes one: without a scene on
+// the device (or if its pool could not be made) the default pool serves.
 cudaError_t scratch_alloc(void **p, size_t bytes, cudaStream_t stream) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
-    if (device < 0 || device >= kMaxDevices) return cudaMallocAsync(p, bytes, stream);
-    cudaMemPool_t pool;
-    if ((e = pool_of(device, &pool)) != cudaSuccess) return e;
-    return cudaMallocFromPoolAsync(p, bytes, pool, stream);
+    cudaMemPool_t pool = nullptr;
+    if (device >= 0 && device < kMaxDevices) {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        if (g_scenes[device] > 0) pool = g_pool[device];
+    }
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : cudaMallocAsync(p, bytes, stream);
 }
 
 cudaError_t scratch_free(void *p, cudaStream_t stream) { return p ? cudaFreeAsync(p, stream) : cudaSuccess; }
 
 void scratch_retain(int device) {
     if (device < 0 || device >= kMaxDevices) return;
-    // the pool exists before any walk, so that none makes it on a capturing stream (a failure here is
-    // reported by the first allocation, which tries again)
-    cudaMemPool_t pool;
-    if (pool_of(device, &pool) != cudaSuccess) cudaGetLastError();
     std::lock_guard<std::mutex> lock(g_mutex);
+    if (!g_pool[device] && make_pool(device) != cudaSuccess) cudaGetLastError();  // (cleared: the default pool serves)
     g_scenes[device]++;
 }
 
