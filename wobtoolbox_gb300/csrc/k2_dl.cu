@@ -227,16 +227,21 @@ cudaError_t launch_min(const SceneView<2> &s, const WalkParams &p_in, const floa
 cudaError_t launch_dl_grid_2d(int min_blocks, const SceneView<2> &s, const WalkParams &p, const float *pts,
                               uint32_t n_points, double *sum, double *sumsq, unsigned long long *bounces,
                               float *per_path, cudaStream_t stream) {
-    // With every warp of the launch resident at 8 blocks per SM, fewer registers only cost spills (64
-    // points x 64 paths: 34 us at 8 blocks, 38 at 12; 1000 points x 200 paths, past the line: 76 and 64).
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (min_blocks > 8 && (uint64_t)n_points * ((p.n_paths + 31u) / 32u) <= (uint64_t)sms * 8u * (kBlock / 32)) min_blocks = 8;
+    if (min_blocks == 0) {
+        // By size: 12 blocks per SM (1024-segment star, 7,960 points x 1024 paths: 2.87 ms against 3.88, 2.95 and
+        // 2.86 at 5, 8 and 10; 8192 segments: 1.23 against 2.00, 1.45 and 1.33). With every warp of the
+        // launch resident at 8 blocks, fewer registers only cost spills (64 points x 64 paths: 34 us at 8
+        // blocks, 38 at 12; 1000 points x 200 paths, past the line: 76 and 64).
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        min_blocks = (uint64_t)n_points * ((p.n_paths + 31u) / 32u) <= (uint64_t)sms * 8u * (kBlock / 32) ? 8 : 12;
+    }
     switch (min_blocks) {
+    case 1: return launch_min<1>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
     case 5: return launch_min<5>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
+    case 6: return launch_min<6>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
     case 8: return launch_min<8>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
-    case 10: return launch_min<10>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
     default: return launch_min<12>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
     }
 }

@@ -11,26 +11,24 @@ namespace wobgb {
 
 // ---- autotuned variants: 0 = 3D direct uniform, 1 = 2D double-layer line intersection,
 // 2 = 3D direct Neumann, 3 = 3D forward single-layer Neumann; configuration c = kernel shape
-// (c % 4: for variants 0-2 the minimum resident blocks {5, 8, 10, 12}; for variant 3 the
+// (c % 4: for variants 0-2 the minimum resident blocks {1 (no limit), 5, 6, 8}; for variant 3 the
 // lockstep kernel at >= 5 blocks/SM or the split-phase wavefront k_fwd_wave.cu in its three trace
 // shapes) and c / 4: paths-per-lane cap {launcher's choice (up to 8), 4, 2, 1} for the lockstep
 // kernels, paths per wavefront chunk {2^22, 2^21, 2^20, 2^19} for the wavefront.
 namespace {
-// Defaults, each the fastest of its configurations over sizes: the 3D direct walks at >= 8 blocks/SM
-// (81,920-triangle Robin slice, 512 paths: 24.4 ms against 25.0 at >= 5, 36.0 at >= 10 and, before, 37.8
-// without a register cap; direct Neumann on 81,920 triangles: 3.97 ms against 4.39, 4.01 and 4.52),
-// the 2D double layer at >= 12 (1024-segment star: 2.87 ms against 3.88, 2.95 and 2.86 at >= 5, 8 and 10;
-// 8192 segments: 1.23 against 2.00, 1.45 and 1.33), the 3D forward walk on the wavefront (trace at >= 9 blocks/SM on
-// compressed nodes, 2^22-path chunks).
-const int kDefaultConfig[kNumTunable] = {1, 3, 1, 3};
+// Defaults: the 3D direct walks at >= 8 blocks/SM (81,920-triangle Robin slice, 512 paths: 24.4 ms against
+// 25.0 at >= 5, 36.0 at >= 10 and 37.8 without a register cap; direct Neumann on 81,920 triangles: 3.97 ms
+// against 4.39, 4.01 and 4.52), the 2D double layer by size (launch_dl_grid_2d), the 3D forward walk on the
+// wavefront (trace at >= 9 blocks/SM on compressed nodes, 2^22-path chunks).
+const int kDefaultConfig[kNumTunable] = {3, 3, 3, 3};
 std::atomic<int> g_config[kNumTunable] = {{-1}, {-1}, {-1}, {-1}};  // -1: the default
 const char *kFwdNames[kTuneOccupancies] = {"lockstep walk, >=5 blocks/SM", "wavefront, trace >=8 blocks/SM",
                                            "wavefront, trace >=6 blocks/SM",
                                            "wavefront, trace >=9 blocks/SM, 64-byte compressed nodes"};
 const uint32_t kWaveSlotsOf[kTunePptCaps] = {1u << 22, 1u << 21, 1u << 20, 1u << 19};
-const int kMinBOf[kTuneOccupancies] = {5, 8, 10, 12};
+const int kMinBOf[kTuneOccupancies] = {1, 5, 6, 8};
 const uint32_t kPptCapOf[kTunePptCaps] = {0u, 4u, 2u, 1u};
-const char *kOccNames[kTuneOccupancies] = {">=5 blocks/SM", ">=8 blocks/SM", ">=10 blocks/SM", ">=12 blocks/SM"};
+const char *kOccNames[kTuneOccupancies] = {"no register cap", ">=5 blocks/SM", ">=6 blocks/SM", ">=8 blocks/SM"};
 const char *kPptNames[kTunePptCaps] = {"paths/lane <= 8", "paths/lane <= 4", "paths/lane <= 2", "paths/lane = 1"};
 char g_names[kTuneConfigs][64];
 }  // namespace
@@ -80,9 +78,9 @@ static cudaError_t launch_cfg(int config, const SceneView<D> &s, const WalkParam
     p.ppt_cap = kPptCapOf[config / kTuneOccupancies];
     switch (kMinBOf[config % kTuneOccupancies]) {
     case 5: return launch_domain_variant<D, kBie, kStrat, false, 5>(s, p, pts, n, sum, sumsq, b, pp, st);
+    case 6: return launch_domain_variant<D, kBie, kStrat, false, 6>(s, p, pts, n, sum, sumsq, b, pp, st);
     case 8: return launch_domain_variant<D, kBie, kStrat, false, 8>(s, p, pts, n, sum, sumsq, b, pp, st);
-    case 10: return launch_domain_variant<D, kBie, kStrat, false, 10>(s, p, pts, n, sum, sumsq, b, pp, st);
-    default: return launch_domain_variant<D, kBie, kStrat, false, 12>(s, p, pts, n, sum, sumsq, b, pp, st);
+    default: return launch_domain_variant<D, kBie, kStrat, false, 1>(s, p, pts, n, sum, sumsq, b, pp, st);
     }
 }
 
@@ -98,8 +96,10 @@ cudaError_t launch_domain_config(int dim, int variant, int config, const void *s
         const SceneView<2> &v = *(const SceneView<2> *)scene_view;
         WalkParams q = p;
         q.ppt_cap = kPptCapOf[config / kTuneOccupancies];
-        if (v.lg_K != 0u)
-            return launch_dl_grid_2d(kMinBOf[config % kTuneOccupancies], v, q, pts, n, sum, sumsq, b, pp, st);
+        if (v.lg_K != 0u) {
+            const int min_blocks = g_config[1].load() < 0 ? 0 : kMinBOf[config % kTuneOccupancies];
+            return launch_dl_grid_2d(min_blocks, v, q, pts, n, sum, sumsq, b, pp, st);
+        }
         return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 8>(v, q, pts, n, sum, sumsq, b, pp, st);
     }
     if (variant == 2 && dim == 3)

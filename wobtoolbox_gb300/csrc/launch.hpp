@@ -113,7 +113,7 @@ cudaError_t launch_fwd_wave_3d(const SceneView<3> &s, const WalkParams &p, const
                                double *sum, double *sumsq, unsigned long long *bounces, float *per_path, int shape,
                                uint32_t max_slots, cudaStream_t stream);
 // The 2D double-layer Dirichlet walk on a scene with a line grid, queries shared by the warp (k2_dl.cu),
-// compiled for min_blocks (5, 8, 10 or 12) resident blocks per SM.
+// compiled for min_blocks (1, 5, 6, 8 or 12) resident blocks per SM; 0: chosen by the launch's size.
 cudaError_t launch_dl_grid_2d(int min_blocks, const SceneView<2> &s, const WalkParams &p, const float *pts,
                               uint32_t n_points, double *sum, double *sumsq, unsigned long long *bounces,
                               float *per_path, cudaStream_t stream);
