@@ -174,8 +174,11 @@ int wob_solve_domain_host(wob_scene scene, const wob_params *params, const float
  * the specialised walk kernels are compiled for several occupancy targets (minimum resident
  * blocks per SM 1, 5, 6, 8) and run with a cap on the paths one lane takes per warp unit (the
  * launcher's choice up to 8, or 4, 2, 1) -- WOB_TUNE_CONFIGS configurations, index = occupancy +
- * 4 x cap; the 3D forward single-layer walk's shapes are the lockstep kernel and the split-phase
- * wavefront's three trace shapes, its second index the wavefront's chunk size. This times each on
+ * 4 x cap; the 2D double layer's last occupancy is 8 for launches that are resident at 8 blocks and
+ * 12 for larger ones; the 3D forward single-layer walk's shapes are the lockstep kernel and the
+ * split-phase wavefront's three trace shapes, its second index the wavefront's chunk size, and its
+ * index 3 takes the lockstep kernel for launches that are resident there (97,280 paths on 152 SMs).
+ * Index 3 is what every variant starts with. This times each on
  * the first points (device pointer, about 2^23 paths, the paths per lane that a launch over all
  * n_points would take) with the given parameters and makes the fastest the one used for that
  * kernel variant from then on
@@ -191,7 +194,8 @@ int wob_autotune_domain(wob_scene scene, const wob_params *params, const float *
 
 /* The tunable kernel variant a solve with these parameters uses (-1: none). */
 int wob_tunable_variant(wob_scene scene, const wob_params *params, int32_t *variant);
-/* Fix / read the configuration of a tunable variant (e.g. to reuse an earlier tuning result). */
+/* Fix / read the configuration of a tunable variant (e.g. to reuse an earlier tuning result; setting
+ * the one that was read restores the variant's state). */
 int wob_set_domain_config(int32_t variant, int32_t config);
 int wob_get_domain_config(int32_t variant, int32_t *config);
 

@@ -11,17 +11,18 @@ namespace wobgb {
 
 // ---- autotuned variants: 0 = 3D direct uniform, 1 = 2D double-layer line intersection,
 // 2 = 3D direct Neumann, 3 = 3D forward single-layer Neumann; configuration c = kernel shape
-// (c % 4: for variants 0-2 the minimum resident blocks {1 (no limit), 5, 6, 8}; for variant 3 the
-// lockstep kernel at >= 5 blocks/SM or the split-phase wavefront k_fwd_wave.cu in its three trace
-// shapes) and c / 4: paths-per-lane cap {launcher's choice (up to 8), 4, 2, 1} for the lockstep
-// kernels, paths per wavefront chunk {2^22, 2^21, 2^20, 2^19} for the wavefront.
+// (c % 4: for variants 0-2 the minimum resident blocks {1 (no limit), 5, 6, 8}, the last of variant 1
+// going on to 12 by size; for variant 3 the lockstep kernel at >= 5 blocks/SM or the split-phase
+// wavefront k_fwd_wave.cu in its three trace shapes) and c / 4: paths-per-lane cap {launcher's choice
+// (up to 8), 4, 2, 1} for the lockstep kernels, paths per wavefront chunk {2^22, 2^21, 2^20, 2^19} for
+// the wavefront. Every variant starts with configuration kDefaultConfig, and what a configuration runs
+// depends on nothing else, so setting the one that was read restores the state.
 namespace {
-// Defaults: the 3D direct walks at >= 8 blocks/SM (81,920-triangle Robin slice, 512 paths: 24.4 ms against
-// 25.0 at >= 5, 36.0 at >= 10 and 37.8 without a register cap; direct Neumann on 81,920 triangles: 3.97 ms
-// against 4.39, 4.01 and 4.52), the 2D double layer by size (launch_dl_grid_2d), the 3D forward walk on the
-// wavefront (trace at >= 9 blocks/SM on compressed nodes, 2^22-path chunks).
-const int kDefaultConfig[kNumTunable] = {3, 3, 3, 3};
-std::atomic<int> g_config[kNumTunable] = {{-1}, {-1}, {-1}, {-1}};  // -1: the default
+// 81,920-triangle Robin slice, 512 paths: 24.4 ms at >= 8 blocks/SM, 25.0 at >= 5, 36.0 at >= 10, 37.8 without
+// a register cap; direct Neumann on 81,920 triangles: 3.97 ms against 4.39, 4.01 and 4.52. 2D double layer:
+// launch_dl_grid_2d. 3D forward: launch_forward_3d.
+constexpr int kDefaultConfig = 3;
+std::atomic<int> g_config[kNumTunable] = {{kDefaultConfig}, {kDefaultConfig}, {kDefaultConfig}, {kDefaultConfig}};
 const char *kFwdNames[kTuneOccupancies] = {"lockstep walk, >=5 blocks/SM", "wavefront, trace >=8 blocks/SM",
                                            "wavefront, trace >=6 blocks/SM",
                                            "wavefront, trace >=9 blocks/SM, 64-byte compressed nodes"};
@@ -42,16 +43,11 @@ int tunable_domain_variant(int dim, const WalkParams &p) {
     if (dim == 3 && st == kStratFwdSlNeumann) return 3;
     return -1;
 }
-int domain_config(int variant) {
-    if (variant < 0 || variant >= kNumTunable) return 0;
-    const int c = g_config[variant].load();
-    return c >= 0 ? c : kDefaultConfig[variant];
-}
+int domain_config(int variant) { return (variant >= 0 && variant < kNumTunable) ? g_config[variant].load() : 0; }
 void set_domain_config(int variant, int config) {
     if (variant >= 0 && variant < kNumTunable && config >= 0 && config < kTuneConfigs) g_config[variant].store(config);
 }
 const char *domain_config_name(int variant, int config) {
-    (void)variant;
     if (config < 0 || config >= kTuneConfigs) return "";
     static char fwd_names[kTuneConfigs][80];
     if (variant == 3) {
@@ -84,6 +80,27 @@ static cudaError_t launch_cfg(int config, const SceneView<D> &s, const WalkParam
     }
 }
 
+// Configuration 3 chooses by size: a forward walk whose warps are all resident in the lockstep kernel (5
+// blocks per SM, 97,280 paths) takes that, since the wavefront's phases then have too few paths to fill
+// (327,680 triangles, 4 bounces: 64,000 paths 0.85 ms lockstep, 1.07 wavefront; 128,000 paths 1.49 and
+// 1.27); larger ones take the wavefront on compressed nodes, as 7, 11 and 15 do at every size.
+static cudaError_t launch_forward_3d(int config, const SceneView<3> &s, const WalkParams &p, const float *pts, uint32_t n,
+                                     double *sum, double *sumsq, unsigned long long *b, float *pp, cudaStream_t st) {
+    WalkParams q = p;
+    q.ppt_cap = kPptCapOf[config / kTuneOccupancies];
+    const int shape = config % kTuneOccupancies;
+    bool lockstep = shape == 0 || p.no_alloc;
+    if (config == 3) {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        lockstep = lockstep || (uint64_t)n * ((p.n_paths + 31u) / 32u) <= (uint64_t)sms * 5u * (kWalkBlock / 32);
+    }
+    if (lockstep)
+        return launch_domain_variant<3, kSingleLayer, kStratFwdSlNeumann, false, 5>(s, q, pts, n, sum, sumsq, b, pp, st);
+    return launch_fwd_wave_3d(s, p, pts, n, sum, sumsq, b, pp, shape, kWaveSlotsOf[config / kTuneOccupancies], st);
+}
+
 cudaError_t launch_domain_config(int dim, int variant, int config, const void *scene_view, const WalkParams &p,
                                  const float *pts, uint32_t n, double *sum, double *sumsq, unsigned long long *b,
                                  float *pp, cudaStream_t st) {
@@ -97,22 +114,15 @@ cudaError_t launch_domain_config(int dim, int variant, int config, const void *s
         WalkParams q = p;
         q.ppt_cap = kPptCapOf[config / kTuneOccupancies];
         if (v.lg_K != 0u) {
-            const int min_blocks = g_config[1].load() < 0 ? 0 : kMinBOf[config % kTuneOccupancies];
+            const int min_blocks = config % kTuneOccupancies == 3 ? 0 : kMinBOf[config % kTuneOccupancies];
             return launch_dl_grid_2d(min_blocks, v, q, pts, n, sum, sumsq, b, pp, st);
         }
         return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 8>(v, q, pts, n, sum, sumsq, b, pp, st);
     }
     if (variant == 2 && dim == 3)
         return launch_cfg<3, kDirect, kStratDirectNeumann>(config, *(const SceneView<3> *)scene_view, p, pts, n, sum, sumsq, b, pp, st);
-    if (variant == 3 && dim == 3) {
-        WalkParams q = p;
-        q.ppt_cap = kPptCapOf[config / kTuneOccupancies];
-        const SceneView<3> &v = *(const SceneView<3> *)scene_view;
-        const int shape = config % kTuneOccupancies;
-        if (shape == 0 || p.no_alloc)
-            return launch_domain_variant<3, kSingleLayer, kStratFwdSlNeumann, false, 5>(v, q, pts, n, sum, sumsq, b, pp, st);
-        return launch_fwd_wave_3d(v, p, pts, n, sum, sumsq, b, pp, shape, kWaveSlotsOf[config / kTuneOccupancies], st);
-    }
+    if (variant == 3 && dim == 3)
+        return launch_forward_3d(config, *(const SceneView<3> *)scene_view, p, pts, n, sum, sumsq, b, pp, st);
     return cudaErrorInvalidValue;
 }
 
@@ -135,18 +145,7 @@ cudaError_t launch_domain_3d(const SceneView<3> &s, const WalkParams &p, const f
                              double *sum, double *sumsq, unsigned long long *bounces, float *per_path,
                              cudaStream_t stream) {
     const int v = tunable_domain_variant(3, p);
-    int config = domain_config(v);
-    if (v == 3 && g_config[3].load() < 0) {
-        // Unless a configuration was chosen: a forward walk whose warps are all resident in the lockstep
-        // kernel (5 blocks per SM, 97,280 paths) takes that; the wavefront's phases then have too few
-        // paths to fill (327,680 triangles, 4 bounces: 64,000 paths 0.85 ms lockstep, 1.07 wavefront;
-        // 128,000 paths 1.49 and 1.27).
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if ((uint64_t)n_points * ((p.n_paths + 31u) / 32u) <= (uint64_t)sms * 5u * (kWalkBlock / 32)) config = 0;
-    }
-    if (v >= 0) return launch_domain_config(3, v, config, &s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
+    if (v >= 0) return launch_domain_config(3, v, domain_config(v), &s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
     const int st = strategy_of(p.bie, p.estimator, p.problem);
     if (p.n_volume == 0 && st == kStratSingleLayer)
         return launch_domain_variant<3, kSingleLayer, kStratSingleLayer, false, 5>(s, p, pts, n_points, sum, sumsq, bounces, per_path, stream);
