@@ -75,6 +75,27 @@ def test_published_occupancies(engine, cuda, tmp_path, configure, variant):
     scene.close()
 
 
+@pytest.mark.parametrize("n_seg,points,paths", [(40, 3, 33), (300, 304, 256), (300, 305, 256)])
+def test_double_layer_without_a_line_grid(engine, oracle, cuda, tmp_path, configure, n_seg, points, paths):
+    """Device-built scenes, which have no line grid: each configuration runs its own occupancy (no limit:
+    4), the last one 4 or 8 by size, with the oracle's path values."""
+    torch = cuda
+    sc = S.scene2d(0, False, n_seg=n_seg)
+    t = lambda a, dt=torch.float32: torch.from_numpy(np.ascontiguousarray(a)).to("cuda", dt)  # noqa: E731
+    scene = engine.SceneHost.build_on_device(t(sc["verts"]), t(sc["normals"]), t(sc["bvals"]), t(sc["types"], torch.int32))
+    pts = np.random.default_rng(points).uniform(-0.4, 0.4, (points, 2)).astype(np.float32)
+    p = engine.EstimatorParams(bie_model=1, path_length=3, num_sample_paths=paths, seed=11)
+    small = points * -(-paths // 32) <= 16 * torch.cuda.get_device_properties(0).multi_processor_count
+    ref = oracle.solve_domain(oracle.Elements(*scene.stored_arrays()), p, pts, per_path=True)[3]
+    d = torch.from_numpy(pts).cuda()
+    for config in range(4):
+        configure(1, config)
+        assert launches(torch, tmp_path, scene, p, pts) == [("domain_kernel", (4, 5, 6, 4 if small else 8)[config])]
+        got = _paths(engine, torch, scene, p, d, points)
+        assert ((got == ref) | (np.isnan(got) & np.isnan(ref))).all()
+    scene.close()
+
+
 def test_every_variant_starts_with_configuration_3_and_gets_it_back(engine, cuda, tmp_path):
     """Reading, changing and setting back what was read leaves every later solve's kernels as they were."""
     import subprocess

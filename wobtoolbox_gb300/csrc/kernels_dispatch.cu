@@ -12,7 +12,7 @@ namespace wobgb {
 // ---- autotuned variants: 0 = 3D direct uniform, 1 = 2D double-layer line intersection,
 // 2 = 3D direct Neumann, 3 = 3D forward single-layer Neumann; configuration c = kernel shape
 // (c % 4: for variants 0-2 the minimum resident blocks {1 (no limit), 5, 6, 8}, the last of variant 1
-// going on to 12 by size; for variant 3 the lockstep kernel at >= 5 blocks/SM or the split-phase
+// by the size of the launch; for variant 3 the lockstep kernel at >= 5 blocks/SM or the split-phase
 // wavefront k_fwd_wave.cu in its three trace shapes) and c / 4: paths-per-lane cap {launcher's choice
 // (up to 8), 4, 2, 1} for the lockstep kernels, paths per wavefront chunk {2^22, 2^21, 2^20, 2^19} for
 // the wavefront. Every variant starts with configuration kDefaultConfig, and what a configuration runs
@@ -67,6 +67,14 @@ const char *domain_config_name(int variant, int config) {
     return g_names[config];
 }
 
+// All warps of a launch (32 paths of a point each) are resident at `blocks` blocks per SM.
+static bool resident(uint32_t n_points, uint32_t n_paths, uint32_t blocks) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return (uint64_t)n_points * ((n_paths + 31u) / 32u) <= (uint64_t)sms * blocks * (kWalkBlock / 32);
+}
+
 template <int D, int kBie, int kStrat>
 static cudaError_t launch_cfg(int config, const SceneView<D> &s, const WalkParams &p_in, const float *pts, uint32_t n,
                               double *sum, double *sumsq, unsigned long long *b, float *pp, cudaStream_t st) {
@@ -80,6 +88,23 @@ static cudaError_t launch_cfg(int config, const SceneView<D> &s, const WalkParam
     }
 }
 
+// The double layer without a line grid. By size (0): launches that are resident at 4 blocks per SM take
+// those (64 points x 64 paths on 256 segments: 0.142 ms against 0.153, 0.152 and 0.152 at >= 5, 6 and 8; 2,400
+// warps on 1024: 0.336 against 0.341, 0.358 and 0.343), others 8 (2,800 warps: 0.355 against 0.571 at 4 and
+// 0.359 at 5; 4,000 points x 256 paths on 8192 segments: 7.2 against 11.1, 9.4 and 8.3 at 4, 5 and 6). Without a
+// limit the kernel takes 130 registers, which 3 blocks fit and 4 do not (4,000 x 256 on 1024: 5.0 ms
+// against 3.9 at 4), so "no limit" is 4.
+static cudaError_t launch_dl_2d(int min_blocks, const SceneView<2> &s, const WalkParams &p, const float *pts, uint32_t n,
+                                double *sum, double *sumsq, unsigned long long *b, float *pp, cudaStream_t st) {
+    if (min_blocks == 0) min_blocks = resident(n, p.n_paths, 4) ? 4 : 8;
+    switch (min_blocks) {
+    case 5: return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 5>(s, p, pts, n, sum, sumsq, b, pp, st);
+    case 6: return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 6>(s, p, pts, n, sum, sumsq, b, pp, st);
+    case 8: return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 8>(s, p, pts, n, sum, sumsq, b, pp, st);
+    default: return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 4>(s, p, pts, n, sum, sumsq, b, pp, st);
+    }
+}
+
 // Configuration 3 chooses by size: a forward walk whose warps are all resident in the lockstep kernel (5
 // blocks per SM, 97,280 paths) takes that, since the wavefront's phases then have too few paths to fill
 // (327,680 triangles, 4 bounces: 64,000 paths 0.85 ms lockstep, 1.07 wavefront; 128,000 paths 1.49 and
@@ -89,14 +114,7 @@ static cudaError_t launch_forward_3d(int config, const SceneView<3> &s, const Wa
     WalkParams q = p;
     q.ppt_cap = kPptCapOf[config / kTuneOccupancies];
     const int shape = config % kTuneOccupancies;
-    bool lockstep = shape == 0 || p.no_alloc;
-    if (config == 3) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        lockstep = lockstep || (uint64_t)n * ((p.n_paths + 31u) / 32u) <= (uint64_t)sms * 5u * (kWalkBlock / 32);
-    }
-    if (lockstep)
+    if (shape == 0 || p.no_alloc || (config == 3 && resident(n, p.n_paths, 5)))
         return launch_domain_variant<3, kSingleLayer, kStratFwdSlNeumann, false, 5>(s, q, pts, n, sum, sumsq, b, pp, st);
     return launch_fwd_wave_3d(s, p, pts, n, sum, sumsq, b, pp, shape, kWaveSlotsOf[config / kTuneOccupancies], st);
 }
@@ -113,11 +131,9 @@ cudaError_t launch_domain_config(int dim, int variant, int config, const void *s
         const SceneView<2> &v = *(const SceneView<2> *)scene_view;
         WalkParams q = p;
         q.ppt_cap = kPptCapOf[config / kTuneOccupancies];
-        if (v.lg_K != 0u) {
-            const int min_blocks = config % kTuneOccupancies == 3 ? 0 : kMinBOf[config % kTuneOccupancies];
-            return launch_dl_grid_2d(min_blocks, v, q, pts, n, sum, sumsq, b, pp, st);
-        }
-        return launch_domain_variant<2, kDoubleLayer, kStratLineIntersection, false, 8>(v, q, pts, n, sum, sumsq, b, pp, st);
+        const int min_blocks = config % kTuneOccupancies == 3 ? 0 : kMinBOf[config % kTuneOccupancies];
+        if (v.lg_K != 0u) return launch_dl_grid_2d(min_blocks, v, q, pts, n, sum, sumsq, b, pp, st);
+        return launch_dl_2d(min_blocks, v, q, pts, n, sum, sumsq, b, pp, st);
     }
     if (variant == 2 && dim == 3)
         return launch_cfg<3, kDirect, kStratDirectNeumann>(config, *(const SceneView<3> *)scene_view, p, pts, n, sum, sumsq, b, pp, st);
