@@ -174,8 +174,8 @@ int wob_solve_domain_host(wob_scene scene, const wob_params *params, const float
  * the specialised walk kernels are compiled for several occupancy targets (minimum resident
  * blocks per SM 1, 5, 6, 8) and run with a cap on the paths one lane takes per warp unit (the
  * launcher's choice up to 8, or 4, 2, 1) -- WOB_TUNE_CONFIGS configurations, index = occupancy +
- * 4 x cap; the 2D double layer's last occupancy is chosen by the launch's size (8 or 12 with a line
- * grid, 4 or 8 without); the 3D forward single-layer walk's shapes are the lockstep kernel and the
+ * 4 x cap; the last occupancy is chosen by the launch's size (8, fewer while all its warps are
+ * resident with fewer, 12 for the 2D double layer on a line grid); the 3D forward single-layer walk's shapes are the lockstep kernel and the
  * split-phase wavefront's three trace shapes, its second index the wavefront's chunk size, and its
  * index 3 takes the lockstep kernel for launches that are resident there (97,280 paths on 152 SMs).
  * Index 3 is what every variant starts with. This times each on

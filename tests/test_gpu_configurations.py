@@ -67,11 +67,40 @@ def _variant_case(engine, variant):
 
 @pytest.mark.parametrize("variant", [0, 1, 2])
 def test_published_occupancies(engine, cuda, tmp_path, configure, variant):
-    """Configuration c of the walk kernels: the (c mod 4)-th of 1, 5, 6, 8 resident blocks per SM."""
+    """Configuration c of the walk kernels: the (c mod 4)-th of 1, 5, 6 resident blocks per SM and the one by
+    size; a launch past every line takes 8 (12 for the double layer)."""
+    import dataclasses
     scene, p, pts = _variant_case(engine, variant)
+    large = dataclasses.replace(p, num_sample_paths=30000)
     for config in range(16):
         configure(variant, config)
-        assert launches(cuda, tmp_path, scene, p, pts) == [("dl2d_kernel" if variant == 1 else "domain_kernel", (1, 5, 6, 8)[config % 4])]
+        name = "dl2d_kernel" if variant == 1 else "domain_kernel"
+        assert launches(cuda, tmp_path, scene, p, pts) == [(name, (1, 5, 6, 8 if variant == 1 else 1)[config % 4])]
+        assert launches(cuda, tmp_path, scene, large, pts) == [(name, (1, 5, 6, 12 if variant == 1 else 8)[config % 4])]
+    scene.close()
+
+
+@pytest.mark.parametrize("problem", [1, 3])
+@pytest.mark.parametrize("points,paths", [(456, 128), (457, 128), (760, 128), (761, 128)])
+def test_direct_walks_on_both_sides_of_their_size_rules(engine, oracle, cuda, tmp_path, configure, problem, points, paths):
+    """No cap, 5 and 8 blocks per SM by the launch's size: the oracle's path values, and sums, of each."""
+    torch = cuda
+    sc = S.scene3d(problem, False, subdiv=1)
+    scene = engine.SceneHost(sc["verts"], sc["normals"], sc["bvals"], sc["types"], sc["alphas"])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    pts = np.random.default_rng(points).uniform(-0.3, 0.3, (points, 3)).astype(np.float32)
+    p = engine.EstimatorParams(bie_model=2, problem=problem, path_length=3, num_sample_paths=paths, seed=5)
+    warps = points * -(-paths // 32)
+    variant = 2 if problem == 1 else 0
+    configure(variant, 3)
+    want = 1 if warps <= 12 * sms else 5 if warps <= 20 * sms else 8
+    assert launches(torch, tmp_path, scene, p, pts) == [("domain_kernel", want)]
+    ref = oracle.solve_domain(oracle.Elements(*scene.stored_arrays()), p, pts, per_path=True)[3]
+    d = torch.from_numpy(pts).cuda()
+    for config in (3, 2):
+        configure(variant, config)
+        got = _paths(engine, torch, scene, p, d, points)
+        assert ((got == ref) | (np.isnan(got) & np.isnan(ref))).all()
     scene.close()
 
 
@@ -113,7 +142,7 @@ def test_every_variant_starts_with_configuration_3_and_gets_it_back(engine, cuda
         "    old = C.c_int32(-7); wob.check(lib.wob_get_domain_config(v, C.byref(old))); assert old.value == 3, old.value\n"
         "    wob.check(lib.wob_set_domain_config(v, 14)); wob.check(lib.wob_set_domain_config(v, old.value))\n"
         "assert seen() == first, (seen(), first)\n"
-        "assert [f[0][1] for f in first] == [8, 8, 8, 5] and [len(f) for f in first] == [1] * 4, first\n"
+        "assert [f[0][1] for f in first] == [1, 8, 1, 5] and [len(f) for f in first] == [1] * 4, first\n"
         "for c in (-1, 16): assert lib.wob_set_domain_config(0, c) != 0\n"
         "print('restored')\n")
     import os

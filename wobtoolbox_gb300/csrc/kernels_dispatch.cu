@@ -11,8 +11,8 @@ namespace wobgb {
 
 // ---- autotuned variants: 0 = 3D direct uniform, 1 = 2D double-layer line intersection,
 // 2 = 3D direct Neumann, 3 = 3D forward single-layer Neumann; configuration c = kernel shape
-// (c % 4: for variants 0-2 the minimum resident blocks {1 (no limit), 5, 6, 8}, the last of variant 1
-// by the size of the launch; for variant 3 the lockstep kernel at >= 5 blocks/SM or the split-phase
+// (c % 4: for variants 0-2 the minimum resident blocks {1 (no limit), 5, 6, 8 or by the size of the
+// launch}; for variant 3 the lockstep kernel at >= 5 blocks/SM or the split-phase
 // wavefront k_fwd_wave.cu in its three trace shapes) and c / 4: paths-per-lane cap {launcher's choice
 // (up to 8), 4, 2, 1} for the lockstep kernels, paths per wavefront chunk {2^22, 2^21, 2^20, 2^19} for
 // the wavefront. Every variant starts with configuration kDefaultConfig, and what a configuration runs
@@ -75,12 +75,18 @@ static bool resident(uint32_t n_points, uint32_t n_paths, uint32_t blocks) {
     return (uint64_t)n_points * ((n_paths + 31u) / 32u) <= (uint64_t)sms * blocks * (kWalkBlock / 32);
 }
 
+// The 3D direct walks. By size (the last occupancy): launches that are resident without a register cap (3
+// blocks per SM) take no cap, those resident at 5 blocks these, others 8. 20,480 triangles, no cap / 5 / 8: direct
+// Neumann 300 points x 100 paths 0.88 / 0.88 / 0.96 ms, 600 x 128 1.65 / 1.06 / 1.10, 1000 x 128
+// 2.45 / 1.95 / 1.45; mixed data 0.046 / 0.046 / 0.052, 0.085 / 0.056 / 0.062, 0.124 / 0.097 / 0.087.
 template <int D, int kBie, int kStrat>
 static cudaError_t launch_cfg(int config, const SceneView<D> &s, const WalkParams &p_in, const float *pts, uint32_t n,
                               double *sum, double *sumsq, unsigned long long *b, float *pp, cudaStream_t st) {
     WalkParams p = p_in;
     p.ppt_cap = kPptCapOf[config / kTuneOccupancies];
-    switch (kMinBOf[config % kTuneOccupancies]) {
+    int min_blocks = kMinBOf[config % kTuneOccupancies];
+    if (config % kTuneOccupancies == 3) min_blocks = resident(n, p.n_paths, 3) ? 1 : resident(n, p.n_paths, 5) ? 5 : 8;
+    switch (min_blocks) {
     case 5: return launch_domain_variant<D, kBie, kStrat, false, 5>(s, p, pts, n, sum, sumsq, b, pp, st);
     case 6: return launch_domain_variant<D, kBie, kStrat, false, 6>(s, p, pts, n, sum, sumsq, b, pp, st);
     case 8: return launch_domain_variant<D, kBie, kStrat, false, 8>(s, p, pts, n, sum, sumsq, b, pp, st);
