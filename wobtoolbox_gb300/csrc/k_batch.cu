@@ -1,7 +1,8 @@
 // Batched walk: many scenes, each with its own parameters and evaluation points, in one persistent
-// launch per walk class (at most five: backward single layer and forward single-layer Neumann, each
-// with and without a source term, and the general walk, whose code for every model and estimator
-// stalls on instruction fetches: 2.2 cycles an instruction where the sources ran in it). A device table holds, per scene, its scene view, walk parameters and first
+// launch per walk class (at most seven: backward single layer, forward single-layer Neumann and direct with
+// uniform samples, each with and without a source term, and the general walk, whose code for every
+// model and estimator stalls on instruction fetches: 2.2 cycles an instruction where the sources ran
+// in it). A device table holds, per scene, its scene view, walk parameters and first
 // work unit; warps take units in a grid-stride loop and find their scene by bisection over the
 // units' prefix. A unit is 32 * ppt paths of one point of one scene, so a warp never mixes scenes,
 // and the per-scene work is exactly what a single-scene launch does (same walker variant, same
@@ -120,19 +121,23 @@ cudaError_t launch_batch_impl(const BatchEntry<D> *table, uint32_t n_scenes, uin
                               uint64_t path_offset_add, cudaStream_t stream) {
     if (total_units == 0 || n_scenes == 0) return cudaSuccess;
     if (cls == 1u)
-        return launch_class<D, Walker<D, kSingleLayer, kStratSingleLayer, false, true>>(table, n_scenes, total_units, pts, sum,
-                                                                                   sumsq, bounces, path_offset_add, stream);
+        return launch_class<D, Walker<D, kSingleLayer, kStratSingleLayer, false, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
+                                                            path_offset_add, stream);
     if (cls == 2u)
-        return launch_class<D, Walker<D, kSingleLayer, kStratFwdSlNeumann, false, true>>(table, n_scenes, total_units, pts,
-                                                                                    sum, sumsq, bounces, path_offset_add,
-                                                                                    stream);
+        return launch_class<D, Walker<D, kSingleLayer, kStratFwdSlNeumann, false, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
+                                                            path_offset_add, stream);
     if (cls == 3u)
-        return launch_class<D, Walker<D, kSingleLayer, kStratSingleLayer, true, true>>(table, n_scenes, total_units, pts, sum,
-                                                                                  sumsq, bounces, path_offset_add, stream);
+        return launch_class<D, Walker<D, kDirect, kStratUniform, false, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
+                                                            path_offset_add, stream);
     if (cls == 4u)
-        return launch_class<D, Walker<D, kSingleLayer, kStratFwdSlNeumann, true, true>>(table, n_scenes, total_units, pts,
-                                                                                   sum, sumsq, bounces, path_offset_add,
-                                                                                   stream);
+        return launch_class<D, Walker<D, kSingleLayer, kStratSingleLayer, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
+                                                            path_offset_add, stream);
+    if (cls == 5u)
+        return launch_class<D, Walker<D, kSingleLayer, kStratFwdSlNeumann, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
+                                                            path_offset_add, stream);
+    if (cls == 6u)
+        return launch_class<D, Walker<D, kDirect, kStratUniform, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
+                                                            path_offset_add, stream);
     return launch_class<D, Walker<D, -1, kStratRuntime, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
                                                                 path_offset_add, stream);
 }
