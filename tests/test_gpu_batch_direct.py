@@ -1,4 +1,4 @@
-"""Batched scenes of the direct model, with and without a source term, among others: every scene's sums are
+"""Batched scenes of the direct model, with and without a source term, and of the forward estimator, among others: every scene's sums are
 those of its own solve (the same paths, whose values the oracle tests cover, in another order)."""
 from __future__ import annotations
 
@@ -18,14 +18,17 @@ def test_direct_scenes_in_a_batch(engine, oracle, cuda, dim, points, paths):
         (lambda problem, k: S.scene3d(problem, False, subdiv=1 + k % 2, seed=k))
     scenes, params = [], []
     rng = np.random.default_rng(dim)
-    # (model, problem, source): uniform samples (0, 2, 3), line queries (1), other models between them
-    for k, (bie, problem, vol) in enumerate([(2, 0, 0), (2, 2, 1), (0, 2, 0), (2, 3, 0), (2, 1, 0), (1, 0, 0), (2, 3, 1), (2, 0, 1)]):
+    # (model, problem, source, estimator): uniform samples (problems 0, 2, 3), line queries (1), other models and
+    # the forward estimator between them
+    for k, (bie, problem, vol, est) in enumerate([(2, 0, 0, 0), (2, 2, 1, 0), (0, 2, 0, 0), (2, 3, 0, 0), (2, 1, 0, 1),
+                                                  (2, 1, 0, 0), (1, 0, 0, 0), (2, 3, 1, 0), (2, 3, 1, 1), (2, 0, 1, 0),
+                                                  (0, 0, 1, 1), (1, 0, 0, 1), (0, 1, 0, 1)]):
         sc = make(problem, k)
         h = engine.SceneHost(sc["verts"], sc["normals"], sc["bvals"], sc["types"], sc["alphas"])
         if vol:
             h.set_volume_cache(8, 2.6, rng.standard_normal(8 ** dim).astype(np.float32))
         scenes.append(h)
-        params.append(engine.EstimatorParams(bie_model=bie, problem=problem, path_length=4, num_sample_paths=paths, seed=k,
+        params.append(engine.EstimatorParams(bie_model=bie, problem=problem, estimator=est, path_length=4, num_sample_paths=paths, seed=k,
                                              num_volume_samples=vol, num_resampling_candidates=4, eps=1e-5))
     n = len(scenes)
     pts = torch.from_numpy(rng.uniform(-0.3, 0.3, (n * points, dim)).astype(np.float32)).cuda()

@@ -1,8 +1,8 @@
 // Batched walk: many scenes, each with its own parameters and evaluation points, in one persistent
-// launch per walk class (at most seven: backward single layer, forward single-layer Neumann and direct with
-// uniform samples, each with and without a source term, and the general walk, whose code for every
-// model and estimator stalls on instruction fetches: 2.2 cycles an instruction where the sources ran
-// in it). A device table holds, per scene, its scene view, walk parameters and first
+// launch per walk class (at most eight: backward single layer, forward single-layer Neumann and direct with
+// uniform samples, each with and without a source term, the forward estimator's other cases, and the
+// general walk, whose code for every model and estimator stalls on instruction fetches: 2.2 cycles
+// an instruction where the sources ran in it). A device table holds, per scene, its scene view, walk parameters and first
 // work unit; warps take units in a grid-stride loop and find their scene by bisection over the
 // units' prefix. A unit is 32 * ppt paths of one point of one scene, so a warp never mixes scenes,
 // and the per-scene work is exactly what a single-scene launch does (same walker variant, same
@@ -11,7 +11,11 @@
 
 namespace wobgb {
 
-constexpr int kBatchMinB = 6;  // 24 scenes: 11.1 ms at 5, 10.5 at 6, 10.8 at 8
+constexpr int kBatchMinB = 6;     // 24 scenes: 11.1 ms at 5, 10.5 at 6, 10.8 at 8
+// Three scenes, 3,000 points x 128 paths each: direct with a source at 4 (3D mixed data 1.45 ms, 1.80 at 5, 1.36
+// without a cap; Robin 0.49, 0.45, 0.58), the forward estimator at 5 (direct with a source, 3D mixed 0.65 ms,
+// 0.65 at 4, 0.83 in the general walk at 6; 2D 0.50, 0.61, 0.68).
+constexpr int kBatchMinBSource = 4, kBatchMinBForward = 5;
 
 // One unit (32 * ppt paths of one point) of a batched scene with the walker variant W; view and
 // p are the scene's view and parameters staged in shared memory by the warp.
@@ -61,8 +65,8 @@ __device__ __forceinline__ void batch_unit(const BatchEntry<D> &e, const SceneVi
 // One persistent launch per walk class: every scene of the launch runs the same walker variant
 // (the specialisation a single-scene launch of that class uses); a warp finds its scene by
 // bisection over the units' prefix.
-template <int D, class W>
-__global__ void __launch_bounds__(kBlock, kBatchMinB) batch_domain_kernel(const BatchEntry<D> *__restrict__ table,
+template <int D, class W, int kMinB>
+__global__ void __launch_bounds__(kBlock, kMinB) batch_domain_kernel(const BatchEntry<D> *__restrict__ table,
                                                               uint32_t n_scenes, uint64_t total_units,
                                                               const float *__restrict__ pts, double *__restrict__ sum,
                                                               double *__restrict__ sumsq,
@@ -105,11 +109,11 @@ __global__ void __launch_bounds__(kBlock, kBatchMinB) batch_domain_kernel(const 
     }
 }
 
-template <int D, class W>
+template <int D, class W, int kMinB = kBatchMinB>
 cudaError_t launch_class(const BatchEntry<D> *table, uint32_t n_scenes, uint64_t total_units, const float *pts,
                          double *sum, double *sumsq, unsigned long long *bounces, uint64_t path_offset_add,
                          cudaStream_t stream) {
-    auto k = batch_domain_kernel<D, W>;
+    auto k = batch_domain_kernel<D, W, kMinB>;
     k<<<persistent_grid(k, total_units), kBlock, 0, stream>>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
                                                                 path_offset_add);
     return cudaGetLastError();
@@ -136,8 +140,11 @@ cudaError_t launch_batch_impl(const BatchEntry<D> *table, uint32_t n_scenes, uin
         return launch_class<D, Walker<D, kSingleLayer, kStratFwdSlNeumann, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
                                                             path_offset_add, stream);
     if (cls == 6u)
-        return launch_class<D, Walker<D, kDirect, kStratUniform, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
-                                                            path_offset_add, stream);
+        return launch_class<D, Walker<D, kDirect, kStratUniform, true, true>, kBatchMinBSource>(
+            table, n_scenes, total_units, pts, sum, sumsq, bounces, path_offset_add, stream);
+    if (cls == 7u)
+        return launch_class<D, Walker<D, -1, kStratFwdUniform, true, true>, kBatchMinBForward>(
+            table, n_scenes, total_units, pts, sum, sumsq, bounces, path_offset_add, stream);
     return launch_class<D, Walker<D, -1, kStratRuntime, true, true>>(table, n_scenes, total_units, pts, sum, sumsq, bounces,
                                                                 path_offset_add, stream);
 }

@@ -685,14 +685,15 @@ template <int D> struct BatchEntry {
 
 // The specialised walk a batched scene runs: 1 = backward single layer, 2 = forward single-layer
 // Neumann, 3 = direct with uniform samples (data other than all-Neumann), 4 to 6 the same with a source term,
-// 0 = the general walk.
-constexpr uint32_t kBatchClasses = 7u;
+// 7 = the forward estimator's other cases, 0 = the general walk.
+constexpr uint32_t kBatchClasses = 8u;
 __host__ __device__ __forceinline__ uint32_t batch_walk_class(const WalkParams &p) {
     const uint32_t vol = p.n_volume != 0 ? 3u : 0u;
     const int st = strategy_of(p.bie, p.estimator, p.problem);
     if (st == kStratSingleLayer) return 1u + vol;
     if (st == kStratFwdSlNeumann) return 2u + vol;
     if (st == kStratUniform && p.bie == kDirect) return 3u + vol;
+    if (st == kStratFwdUniform) return 7u;
     return 0u;
 }
 
