@@ -4,9 +4,8 @@
 // A query tests the segments its grid cell lists: 5 on average on a 1024-segment star (41 on 8192
 // segments) but up to 40, so a lane per query ran at 13 of 32 lanes and 1,600 instructions a bounce
 // (3.3 ms for 7,960 points x 1024 paths x 8 bounces at 12 blocks per SM; 2.46 ms for 4,000 x 256 on 8192
-// segments). This kernel takes 2.9 ms and 1.23 ms. A
-// warp lays the lists of its 32 queries end to end (a scan of their lengths) and tests 32 candidates at
-// a time, a lane each: the lane finds the query that owns its candidate from the bit mask of the
+// segments). This kernel takes 2.8 ms and 1.23 ms, at 29 lanes and 1,130 instructions. A warp lays the
+// lists of its 32 queries end to end (a scan of their lengths) and tests 32 candidates at a time, a lane each: the lane finds the query that owns its candidate from the bit mask of the
 // queries that begin in the round, fetches that query's line by shuffles, and the round's ballot is
 // kept in shared memory. A query's hits are then a run of ballot bits in list order, so its hit count
 // and the chosen hit are bit counts. The walk's warps stay converged for it: paths that have ended

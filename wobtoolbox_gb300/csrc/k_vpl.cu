@@ -107,8 +107,9 @@ __global__ void __launch_bounds__(32 * kVplSplit) vpl_aggregate3_kernel(const fl
 // they run as the two halves of packed FP32 operations (F2), added to the FP64 sum in tile order. A
 // pair's two quotients and logarithm are the scalar code's, by F2's; pairs outside the packed forms'
 // range (q below eps^2 or beyond 2^60, or a weight out of the quotient's range) take the scalar
-// expressions. The kernel above is bound by issue, 85 instructions a pair; a packed one is issued for
-// two pairs: 100,000 VPLs x 39,280 points 10.2 -> 5.7 ms.
+// expressions. The scalar loop was bound by issue at 95 instructions a pair, a packed instruction is issued
+// for two (45 a pair): 100,000 VPLs x 39,280 points 11.7 -> 7.2 ms, the FMA pipe then at 67 % of its cycles.
+
 // The smaller of two floats, NaN if either is (fminf returns the other one).
 __device__ __forceinline__ float fmin_nan(float a, float b) {
     float m;

@@ -110,12 +110,12 @@ __device__ __forceinline__ float closest_value(const SceneView<2> &s, const Clos
 // which lane runs a path.
 //
 // Queries differ several-fold in length, and with a whole query per loop iteration 9 of 32 lanes were
-// active (9.1 ms for 7,960 points x 256 paths on 1024 segments, issue-bound). Here every lane is in one
-// of three states -- a node to visit, a leaf to test, a finished query -- and the warp executes, each
+// active (8.4 ms for 7,960 points x 256 paths on 1024 segments, issue-bound; 5.2 ms and 14 lanes now). Here
+// every lane is in one of three states -- a node to visit, a leaf to test, a finished query -- and the warp executes, each
 // iteration, the step most of its lanes wait for (finished queries count half: 5.0 ms against 5.4 with
-// equal weights). A query starts from the distance to the previous
-// jump's closest element (where that is finite), which prunes its first descent, and keeps box distances on the stack, so
-// that children the best distance has passed are dropped unvisited; children are ordered by a
+// equal weights when it was chosen). A query starts from the distance to the previous
+// jump's closest element (where that is finite), which prunes its first descent, and keeps box distances
+// on the stack, so that children the best distance has passed are dropped unvisited; children are ordered by a
 // register network. All paths of a point share the first query. The closest element, the
 // lexicographic minimum of (distance, index) over all elements, does not depend on any of this.
 constexpr int kWosShared = 12;  // stack entries in shared memory; deeper ones go to local memory

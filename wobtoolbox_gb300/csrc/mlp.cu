@@ -404,7 +404,7 @@ struct wob_mlp_s {
     // training-loop state (wob_mlp_train)
     uint32_t train_cap = 0, partial_blocks = 0;
     float *xb = nullptr, *tb = nullptr, *sched = nullptr, *partial = nullptr, *partial_loss = nullptr;
-    uint32_t *step = nullptr;   // [2]: step counter, the fused update's count of finished blocks
+    uint32_t *step = nullptr;   // [3]: step counter and the fused step's two notes of it (mlp_train.hpp)
     uint32_t *image = nullptr;  // packed BF16 weights of the fused step (zero padding)
     uint32_t *err = nullptr;    // fused step's error word
     uint32_t inject_wait_polls = 0;  // wob_mlp_inject_wait_timeout

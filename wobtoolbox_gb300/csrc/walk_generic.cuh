@@ -366,9 +366,10 @@ template <int D, int kBie = -1, int kStrat = kStratRuntime, bool kVol = true, bo
     // a time: their D + 1 draws each are a whole number of Philox blocks, cut out of a window of blocks
     // at one position that stays the same from batch to batch (no refill checks, no branches), and
     // their lookups, positions and targets are independent; only the running sum and the selection
-    // are serial. The selection needs no division, and the target's quotients share reciprocals. Against
-    // one candidate at a time: 100,000 paths x 1024 candidates 4.0 -> 3.7 ms, 64 right-hand sides 2.05 ->
-    // 2.00 ms, 24 batched scenes 10.7 -> 10.5 ms.
+    // are serial. The selection needs no division, and the target's quotients share reciprocals.
+    // 100,000 paths x 1024 candidates: 2.2 ms, 4.8 with plain divisions and one record of the guide table
+    // per entry, one candidate at a time. The batches' own part: 64 right-hand sides 2.05 -> 2.00 ms, 24
+    // batched scenes 10.7 -> 10.5 ms.
     static constexpr int kBatch = D == 2 ? 4 : 2;
     __device__ __forceinline__ void ris_select(const BPoint<D> &yp, uint32_t &sel, float *su, float &w_sum,
                                                uint32_t &M) {
